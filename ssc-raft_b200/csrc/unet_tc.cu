@@ -1240,10 +1240,12 @@ int conv3x3_wgrad_tc(const void *dy, const void *x0, int C0, const void *x1, int
     int dev = 0, sms = 148;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    // one CTA per SM over all work items (shared memory holds one), at least
-    // 8 k-blocks each (nine-tap CTAs); two per SM for the row-block kernel
+    // The largest number of pixel ranges whose CTAs run in one wave: shared memory
+    // holds one CTA per SM (164-224 KB), and a CTA past the last SM doubles the
+    // launch (96 -> 32 channels at 8 x 512^2: 1327 us with 150 CTAs).  At least 8
+    // k-blocks per CTA.
     const int items = nine ? Cin / 32 : a.mtiles;
-    long long splits = std::max(1LL, ((nine ? 1LL : 2LL) * sms + items - 1) / items);
+    long long splits = std::max(1, sms / items);
     splits = std::min(splits, std::max(1LL, a.kblocks / 8));
     a.kper = (a.kblocks + splits - 1) / splits;
     a.splits = (int)((a.kblocks + a.kper - 1) / a.kper);
