@@ -22,16 +22,20 @@
 // freshly allocated memory), and all A rows are padded (the reference's
 // padding call is sized by N rows; identical when A == N).
 //
-// B200 design, three kernels per batch of slices, all transforms in shared
-// memory (fft.cuh), no cuFFT and no S x S intermediate in HBM:
+// B200 design, four kernels per batch of slices, all transforms in shared
+// memory (fft.cuh), no cuFFT.  Only the real part of step 6 is used, so the grid
+// enters through its Hermitian part (G(k) + conj G(-k)) / 2: half of its rows, and
+// two image columns per complex transform.
 //   bst_rows_kernel    two projection rows per CTA: pad, filter (the two rows
 //                      as one complex sequence), split, and one complex FFT per
 //                      row carrying both half-rays (separated by symmetry);
 //                      writes only the L/2 radial bins step 5 can read;
-//   bst_regrid_kernel  one Cartesian row per CTA: interpolates the row from
-//                      the polar data straight into shared memory, inverse
-//                      FFT along x, keeps the N crop columns;
-//   bst_cols_kernel    one crop column per CTA: inverse FFT along y, keeps
+//   bst_regrid_kernel  grid rows 0 .. S/2 from the polar data; the geometry of a
+//                      grid point (square root, arc tangent, divisions) is worked
+//                      out once for up to eight slices;
+//   bst_gridrows_kernel  one grid row per CTA: inverse FFT along x, keeps the N
+//                      crop columns;
+//   bst_cols_kernel    two crop columns per CTA: inverse FFT along y, keeps
 //                      the N crop rows, scales.
 // This file is compiled with fast math, as the reference is, so the regrid
 // geometry (hypotf, atan2f, the divisions) follows its rounding.
@@ -56,7 +60,8 @@ namespace {
 struct BstArgs {
     const float *tomo;      // [B][A][N]
     float2 *polar;          // [B][2A][Lh]
-    float2 *T;              // [B][S][N]: rows inverse-transformed along x, crop columns
+    float2 *grid;           // [B][S/2+1][S]: conj of the grid's Hermitian part
+    float2 *T;              // [B][S/2+1][N]: its rows inverse-transformed along x, crop columns
     float *obj;             // [B][N][N]
     FftPlan pN, pL, pS;     // transforms of the filter (Np), the half-rays (L), the grid (S)
     const float2 *G;        // filter weights [Np], or null for 'none'
@@ -65,7 +70,7 @@ struct BstArgs {
     float scale;
 };
 
-// The transforms of the three kernels: NF > 0 is the compile-time length
+// The transforms of the kernels: NF > 0 is the compile-time length
 // that every transform of the launch has (cfft_smem), 0 the plans' lengths.
 template <int NF>
 __device__ __forceinline__ float2 *bst_fft(float2 *a, float2 *b, const FftPlan &P)
@@ -149,63 +154,110 @@ __global__ void __launch_bounds__(512) bst_rows_kernel(const BstArgs p)
     }
 }
 
+// Where a grid point lies in the polar data, and its sign.
+struct GridPoint {
+    size_t q0, q1;        // elements (arc, radius) of the lower and upper arc
+    float pfrac, tfrac;
+    float sgn;            // 0 beyond the last radius
+};
+// array position (X, Y): grid column tx, grid row ty (stored shifted by S/2)
+__device__ __forceinline__ GridPoint grid_point(const BstArgs &p, int X, int Y)
+{
+    const int S = p.S, h = S / 2, twoA = 2 * p.A;
+    const int tx = X - h < 0 ? X - h + S : X - h, ty = Y - h < 0 ? Y - h + S : Y - h;
+    const float posx = (float)(tx - h), posy = (float)(ty - h);
+    const float rho = (float)p.L * hypotf(posx, posy) / (float)S;
+    const float angle = (float)twoA * (0.5f * atan2f(posy, posx) / (float)M_PI + 0.5f);
+    const int irho = (int)rho;
+    int iarc = (int)angle;
+    GridPoint g;
+    g.pfrac = rho - (float)irho;
+    g.tfrac = (float)iarc - angle;
+    // angle lies in [0, twoA] (truncation keeps iarc >= 0): iarc % twoA and
+    // (iarc + 1) % twoA as conditional subtractions
+    iarc = iarc >= twoA ? iarc - twoA : iarc;
+    const int uarc = iarc + 1 >= twoA ? iarc + 1 - twoA : iarc + 1;
+    const bool in = irho < p.L / 2 - 1;
+    g.q0 = in ? (size_t)iarc * p.Lh + irho : 0;
+    g.q1 = in ? (size_t)uarc * p.Lh + irho : 0;
+    g.sgn = in ? 4.f * ((float)(ty & 1) - 0.5f) * ((float)(tx & 1) - 0.5f) : 0.f;
+    return g;
+}
+__device__ __forceinline__ float2 polar_value(const float2 *pol, const GridPoint &g)
+{
+    if (g.sgn == 0.f) return make_float2(0.f, 0.f);
+    const float2 *q0 = pol + g.q0, *q1 = pol + g.q1;
+    const float2 c00 = __ldg(q0), c01 = __ldg(q0 + 1), c10 = __ldg(q1), c11 = __ldg(q1 + 1);
+    const float pf = g.pfrac, tf = g.tfrac;
+    const float2 i0 = make_float2(c00.x * (1.f - pf) + c01.x * pf, c00.y * (1.f - pf) + c01.y * pf);
+    const float2 i1 = make_float2(c10.x * (1.f - pf) + c11.x * pf, c10.y * (1.f - pf) + c11.y * pf);
+    return make_float2((i0.x * tf + i1.x * (1.f - tf)) * g.sgn, (i0.y * tf + i1.y * (1.f - tf)) * g.sgn);
+}
+
+constexpr int kRegridSlices = 8;
+// One thread per grid point of rows 0 .. S/2, for up to eight slices: the point
+// and its mirror image through the origin.  The arithmetic of the two positions
+// (about 200 instructions) is paid once per eight slices; with one grid row and
+// slice per CTA, transformed in place, the kernel was bound by it: 413 us per
+// 2048^2 x 1800 slice (6144 x 6144 points).
+__global__ void __launch_bounds__(256) bst_regrid_kernel(const BstArgs p, int nslices)
+{
+    const int S = p.S, H = S / 2 + 1;
+    const int X = blockIdx.x * 32 + threadIdx.x, Y = blockIdx.y * 8 + threadIdx.y;
+    if (X >= S || Y >= H) return;
+    const GridPoint g = grid_point(p, X, Y), m = grid_point(p, X ? S - X : 0, Y ? S - Y : 0);
+    const int b0 = blockIdx.z * kRegridSlices, b1 = min(b0 + kRegridSlices, nslices);
+    const size_t per = (size_t)2 * p.A * p.Lh, plane = (size_t)H * S;
+    const float2 *pol = p.polar + b0 * per;
+    float2 *out = p.grid + b0 * plane + (size_t)Y * S + X;
+#pragma unroll 4
+    for (int b = b0; b < b1; b++, pol += per, out += plane) {
+        const float2 u = polar_value(pol, g), v = polar_value(pol, m);
+        *out = make_float2(0.5f * (u.x + v.x), 0.5f * (v.y - u.y));   // conj of (u + conj v) / 2
+    }
+}
+
+// T = the forward transform of the conjugated rows: conj of their inverse transform
 template <int NF>
-__global__ void __launch_bounds__(512) bst_regrid_kernel(const BstArgs p)
+__global__ void __launch_bounds__(512) bst_gridrows_kernel(const BstArgs p)
 {
     extern __shared__ float2 sm_bst[];
-    const int slice = blockIdx.y, Y = blockIdx.x;
-    const int S = p.S, h = S / 2, twoA = 2 * p.A;
-    const int ty = (Y - h + S) % S;            // array row Y holds grid row ty (stored shifted by S/2)
-    const float posy = (float)(ty - h);
-    const float sy = 4.f * ((float)(ty % 2) - 0.5f);
-    const float2 *pol = p.polar + (size_t)slice * twoA * p.Lh;
-    const int rmax = p.L / 2 - 1;
-    for (int X = threadIdx.x; X < S; X += blockDim.x) {
-        // (X - h + S) % S, X < S: one conditional add (integer modulos by
-        // run-time values cost about twenty instructions each)
-        const int tx = X - h < 0 ? X - h + S : X - h;
-        const float posx = (float)(tx - h);
-        const float rho = (float)p.L * hypotf(posx, posy) / (float)S;
-        const float angle = (float)twoA * (0.5f * atan2f(posy, posx) / (float)M_PI + 0.5f);
-        const int irho = (int)rho;
-        int iarc = (int)angle;
-        float2 v = make_float2(0.f, 0.f);
-        if (irho < rmax) {
-            const float pfrac = rho - (float)irho;
-            const float tfrac = (float)iarc - angle;
-            // angle lies in [0, twoA] (truncation keeps iarc >= 0): iarc % twoA
-            // and (iarc + 1) % twoA as conditional subtractions
-            iarc = iarc >= twoA ? iarc - twoA : iarc;
-            const int uarc = iarc + 1 >= twoA ? iarc + 1 - twoA : iarc + 1;
-            const float2 *q0 = pol + (size_t)iarc * p.Lh + irho;
-            const float2 *q1 = pol + (size_t)uarc * p.Lh + irho;
-            const float2 c00 = __ldg(q0), c01 = __ldg(q0 + 1), c10 = __ldg(q1), c11 = __ldg(q1 + 1);
-            const float2 i0 = make_float2(c00.x * (1.f - pfrac) + c01.x * pfrac, c00.y * (1.f - pfrac) + c01.y * pfrac);
-            const float2 i1 = make_float2(c10.x * (1.f - pfrac) + c11.x * pfrac, c10.y * (1.f - pfrac) + c11.y * pfrac);
-            v = make_float2(i0.x * tfrac + i1.x * (1.f - tfrac), i0.y * tfrac + i1.y * (1.f - tfrac));
-        }
-        const float sgn = sy * ((float)(tx & 1) - 0.5f);
-        sm_bst[X] = make_float2(v.x * sgn, -v.y * sgn);   // conjugated: see bst_cols_kernel
-    }
+    const int slice = blockIdx.y, Y = blockIdx.x, S = p.S, H = S / 2 + 1;
+    const float2 *row = p.grid + ((size_t)slice * H + Y) * S;
+    for (int X = threadIdx.x; X < S; X += blockDim.x) sm_bst[X] = __ldcs(row + X);
     __syncthreads();
     const float2 *r = bst_fft<NF>(sm_bst, sm_bst + fft_plan_span(p.pS), p.pS);
-    float2 *trow = p.T + ((size_t)slice * S + Y) * p.N;
+    float2 *trow = p.T + ((size_t)slice * H + Y) * p.N;
     for (int i = threadIdx.x; i < p.N; i += blockDim.x) trow[i] = r[p.off + i];
 }
 
-// T holds conj(IFFT_x(grid)); its forward transform along y is the conjugate
-// of the 2-D inverse transform, whose real part is the image.
+// A crop column of T is Hermitian along y (T(S - Y) = conj T(Y)), its forward
+// transform real: columns i and i + 1 are transformed as one complex sequence.
 template <int NF>
 __global__ void __launch_bounds__(512) bst_cols_kernel(const BstArgs p)
 {
     extern __shared__ float2 sm_bst[];
-    const int slice = blockIdx.y, i = blockIdx.x;
-    const float2 *tcol = p.T + (size_t)slice * p.S * p.N + i;
-    for (int Y = threadIdx.x; Y < p.S; Y += blockDim.x) sm_bst[Y] = tcol[(size_t)Y * p.N];
+    const int slice = blockIdx.y, i = 2 * blockIdx.x, S = p.S, H = S / 2 + 1;
+    const bool two = i + 1 < p.N;
+    const float2 *tcol = p.T + (size_t)slice * H * p.N + i;
+    for (int Y = threadIdx.x; Y < H; Y += blockDim.x) {
+        const float2 u = tcol[(size_t)Y * p.N], v = two ? tcol[(size_t)Y * p.N + 1] : make_float2(0.f, 0.f);
+        const int m = Y ? S - Y : 0;
+        if (m == Y) {   // its own mirror image: real
+            sm_bst[Y] = make_float2(u.x, v.x);
+        } else {
+            sm_bst[Y] = make_float2(u.x - v.y, u.y + v.x);
+            sm_bst[m] = make_float2(u.x + v.y, v.x - u.y);
+        }
+    }
     __syncthreads();
     const float2 *r = bst_fft<NF>(sm_bst, sm_bst + fft_plan_span(p.pS), p.pS);
     float *o = p.obj + (size_t)slice * p.N * p.N + i;
-    for (int j = threadIdx.x; j < p.N; j += blockDim.x) o[(size_t)j * p.N] = r[p.off + j].x / p.scale;
+    for (int j = threadIdx.x; j < p.N; j += blockDim.x) {
+        const float2 v = r[p.off + j];
+        o[(size_t)j * p.N] = v.x / p.scale;
+        if (two) o[(size_t)j * p.N + 1] = v.y / p.scale;
+    }
 }
 
 // Forward DFT in FP64 of a 7-smooth length (recursive decimation in time on
@@ -233,11 +285,15 @@ void dft_rec(const std::complex<double> *in, size_t stride, int n, std::complex<
     std::copy(tmp.begin(), tmp.end(), out);
 }
 
+}  // namespace
+
 void dft_host(const std::vector<std::complex<double>> &in, std::vector<std::complex<double>> &out)
 {
     out.assign(in.size(), 0.0);
     dft_rec(in.data(), 1, (int)in.size(), out.data());
 }
+
+namespace {
 
 using BstKey = std::tuple<int, int, int, int, double, double>;
 std::mutex g_bst_mtx;
@@ -366,19 +422,21 @@ bool bst_plan_shape(BstPlanShape &s, int N, int A, int pad)
     return bst_core_ok(c);
 }
 
-size_t bst_workspace_bytes(const BstPlanShape &s, int nslices)
+// Polar rows (later the transformed grid rows in their place) and the half grid.
+static size_t bst_polar_bytes(int A, int Lh, int S, int N, int nslices)
 {
-    const size_t polar = (size_t)nslices * 2 * s.A * s.Lh * sizeof(float2);
-    const size_t T = (size_t)nslices * s.S * s.N * sizeof(float2);
-    return ((polar + 255) & ~(size_t)255) + T;
+    const size_t polar = (size_t)nslices * 2 * A * Lh, T = (size_t)nslices * (S / 2 + 1) * N;
+    return (std::max(polar, T) * sizeof(float2) + 255) & ~(size_t)255;
 }
 
-size_t bst_core_workspace_bytes(const BstCore &c, int nslices)
+static size_t bst_bytes(int A, int Lh, int S, int N, int nslices)
 {
-    const size_t polar = (size_t)nslices * 2 * c.A * c.Lh * sizeof(float2);
-    const size_t T = (size_t)nslices * c.S * c.N * sizeof(float2);
-    return ((polar + 255) & ~(size_t)255) + T;
+    return bst_polar_bytes(A, Lh, S, N, nslices) + (size_t)nslices * (S / 2 + 1) * S * sizeof(float2);
 }
+
+size_t bst_workspace_bytes(const BstPlanShape &s, int nslices) { return bst_bytes(s.A, s.Lh, s.S, s.N, nslices); }
+
+size_t bst_core_workspace_bytes(const BstCore &c, int nslices) { return bst_bytes(c.A, c.Lh, c.S, c.N, nslices); }
 
 // Calls f(integral_constant<int, n>) when n is one of the compiled transform
 // lengths, f(integral_constant<int, 0>) otherwise.
@@ -421,16 +479,21 @@ static void launch_bst_grid(const BstArgs &a, const BstCore &c, int nslices, int
     int dev = 0;
     cudaGetDevice(&dev);
     if (configured != dev) {
-        RAFT_CUDA(cudaFuncSetAttribute(bst_regrid_kernel<NF>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        RAFT_CUDA(cudaFuncSetAttribute(bst_gridrows_kernel<NF>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        (int)kBstSmemMax));
         RAFT_CUDA(cudaFuncSetAttribute(bst_cols_kernel<NF>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        (int)kBstSmemMax));
         configured = dev;
     }
-    bst_regrid_kernel<NF><<<dim3(c.S, nslices), threads, sm2, st>>>(a);
+    const int H = c.S / 2 + 1;
+    bst_regrid_kernel<<<dim3((c.S + 31) / 32, (H + 7) / 8, (nslices + kRegridSlices - 1) / kRegridSlices), dim3(32, 8), 0,
+                        st>>>(a, nslices);
     RAFT_CUDA(cudaGetLastError());
     count_launch();
-    bst_cols_kernel<NF><<<dim3(c.N, nslices), threads, sm2, st>>>(a);
+    bst_gridrows_kernel<NF><<<dim3(H, nslices), threads, sm2, st>>>(a);
+    RAFT_CUDA(cudaGetLastError());
+    count_launch();
+    bst_cols_kernel<NF><<<dim3((c.N + 1) / 2, nslices), threads, sm2, st>>>(a);
     RAFT_CUDA(cudaGetLastError());
 }
 
@@ -443,8 +506,8 @@ void bst_run(int device, const BstCore &c, const float *d_tomo, float *d_obj, in
     BstArgs a;
     a.tomo = d_tomo;
     a.polar = (float2 *)workspace;
-    const size_t polar = (size_t)nslices * 2 * c.A * c.Lh * sizeof(float2);
-    a.T = (float2 *)((char *)workspace + ((polar + 255) & ~(size_t)255));
+    a.T = a.polar;   // the polar rows are read before the grid rows are transformed
+    a.grid = (float2 *)((char *)workspace + bst_polar_bytes(c.A, c.Lh, c.S, c.N, nslices));
     a.obj = d_obj;
     a.G = c.G;
     a.pN = c.G ? fft_table(device, c.Np).plan : FftPlan{};
@@ -464,12 +527,12 @@ void bst_run(int device, const BstCore &c, const float *d_tomo, float *d_obj, in
     const size_t sm3 = 2 * (size_t)a.M * sizeof(float2), sm2 = 2 * (size_t)fft_plan_span(a.pS) * sizeof(float2);
     // compile-time lengths where the plans are direct: the rows kernel's
     // transforms (the filter's, when there is one, and the half-rays') and the
-    // grid transforms of the regrid and column kernels; each kernel then runs
+    // grid transforms of the grid-row and column kernels; each kernel then runs
     // with the thread count of its length
     const bool en = fixed_transforms_enabled();
     const int nrow = (en && a.pL.n == a.pL.M && (!c.G || (a.pN.n == a.pL.n && a.pN.M == a.pN.n))) ? a.pL.n : 0;
     const int ngrid = (en && a.pS.n == a.pS.M) ? a.pS.n : 0;
-    ProfScope ps(PROF_OTHER, st);   // counts the first of the three launches
+    ProfScope ps(PROF_OTHER, st);   // counts the first of the four launches
     with_fixed_length(nrow, [&](auto nf) {
         constexpr int NF = decltype(nf)::value;
         launch_bst_rows<NF>(a, c, nslices, NF ? c_fft_threads(NF) : threads, sm3, st);

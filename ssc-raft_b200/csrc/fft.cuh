@@ -17,6 +17,7 @@
 #include <cuda_runtime.h>
 
 #include <cmath>
+#include <complex>
 #include <vector>
 
 namespace raft {
@@ -520,5 +521,7 @@ struct FftTable {
 const FftTable &fft_table(int device, int n);
 // Transform length the plan of n runs (n, or Bluestein's M); 0 if none fits 24 passes.
 int fft_plan_length(int n);
+// Forward DFT in FP64 on the host (quick for 7-smooth lengths; bst.cu).
+void dft_host(const std::vector<std::complex<double>> &in, std::vector<std::complex<double>> &out);
 
 }  // namespace raft
