@@ -60,12 +60,12 @@ namespace {
 struct BstArgs {
     const float *tomo;      // [B][A][N]
     float2 *polar;          // [B][2A][Lh]
-    float2 *grid;           // [B][S/2+1][S]: conj of the grid's Hermitian part
-    float2 *T;              // [B][S/2+1][N]: its rows inverse-transformed along x, crop columns
+    float2 *grid;           // [B][H][S]: conj of the grid (H = S) or of its Hermitian part (H = S/2+1)
+    float2 *T;              // [B][H][N]: its rows inverse-transformed along x, crop columns
     float *obj;             // [B][N][N]
     FftPlan pN, pL, pS;     // transforms of the filter (Np), the half-rays (L), the grid (S)
     const float2 *G;        // filter weights [Np], or null for 'none'
-    int N, A, Np, L, Lh, S, off, M;   // M = max(Np, L): shared-memory buffer length of the row kernel
+    int N, A, Np, L, Lh, S, H, off, M;   // M = max(Np, L): shared-memory buffer length of the row kernel
     float w_half;           // half-ray weight (the centre sample gets half of it)
     float scale;
 };
@@ -195,25 +195,33 @@ __device__ __forceinline__ float2 polar_value(const float2 *pol, const GridPoint
 }
 
 constexpr int kRegridSlices = 8;
-// One thread per grid point of rows 0 .. S/2, for up to eight slices: the point
-// and its mirror image through the origin.  The arithmetic of the two positions
+// One thread per grid point of rows 0 .. H-1, for up to eight slices: the point
+// and, on the half grid, its mirror image through the origin.  The arithmetic of the two positions
 // (about 200 instructions) is paid once per eight slices; with one grid row and
 // slice per CTA, transformed in place, the kernel was bound by it: 413 us per
 // 2048^2 x 1800 slice (6144 x 6144 points).
+template <bool HALF>
 __global__ void __launch_bounds__(256) bst_regrid_kernel(const BstArgs p, int nslices)
 {
-    const int S = p.S, H = S / 2 + 1;
+    const int S = p.S, H = p.H;
     const int X = blockIdx.x * 32 + threadIdx.x, Y = blockIdx.y * 8 + threadIdx.y;
     if (X >= S || Y >= H) return;
-    const GridPoint g = grid_point(p, X, Y), m = grid_point(p, X ? S - X : 0, Y ? S - Y : 0);
+    const GridPoint g = grid_point(p, X, Y);
+    GridPoint m{};
+    if constexpr (HALF) m = grid_point(p, X ? S - X : 0, Y ? S - Y : 0);
     const int b0 = blockIdx.z * kRegridSlices, b1 = min(b0 + kRegridSlices, nslices);
     const size_t per = (size_t)2 * p.A * p.Lh, plane = (size_t)H * S;
     const float2 *pol = p.polar + b0 * per;
     float2 *out = p.grid + b0 * plane + (size_t)Y * S + X;
 #pragma unroll 4
     for (int b = b0; b < b1; b++, pol += per, out += plane) {
-        const float2 u = polar_value(pol, g), v = polar_value(pol, m);
-        *out = make_float2(0.5f * (u.x + v.x), 0.5f * (v.y - u.y));   // conj of (u + conj v) / 2
+        const float2 u = polar_value(pol, g);
+        if constexpr (HALF) {
+            const float2 v = polar_value(pol, m);
+            *out = make_float2(0.5f * (u.x + v.x), 0.5f * (v.y - u.y));   // conj of (u + conj v) / 2
+        } else {
+            *out = make_float2(u.x, -u.y);
+        }
     }
 }
 
@@ -222,7 +230,7 @@ template <int NF>
 __global__ void __launch_bounds__(512) bst_gridrows_kernel(const BstArgs p)
 {
     extern __shared__ float2 sm_bst[];
-    const int slice = blockIdx.y, Y = blockIdx.x, S = p.S, H = S / 2 + 1;
+    const int slice = blockIdx.y, Y = blockIdx.x, S = p.S, H = p.H;
     const float2 *row = p.grid + ((size_t)slice * H + Y) * S;
     for (int X = threadIdx.x; X < S; X += blockDim.x) sm_bst[X] = __ldcs(row + X);
     __syncthreads();
@@ -231,19 +239,22 @@ __global__ void __launch_bounds__(512) bst_gridrows_kernel(const BstArgs p)
     for (int i = threadIdx.x; i < p.N; i += blockDim.x) trow[i] = r[p.off + i];
 }
 
-// A crop column of T is Hermitian along y (T(S - Y) = conj T(Y)), its forward
+// The image columns are the real parts of the crop columns' forward transforms.
+// HALF: a crop column of T is Hermitian along y (T(S - Y) = conj T(Y)), its
 // transform real: columns i and i + 1 are transformed as one complex sequence.
-template <int NF>
+template <int NF, bool HALF>
 __global__ void __launch_bounds__(512) bst_cols_kernel(const BstArgs p)
 {
     extern __shared__ float2 sm_bst[];
-    const int slice = blockIdx.y, i = 2 * blockIdx.x, S = p.S, H = S / 2 + 1;
-    const bool two = i + 1 < p.N;
+    const int slice = blockIdx.y, i = (HALF ? 2 : 1) * blockIdx.x, S = p.S, H = p.H;
+    const bool two = HALF && i + 1 < p.N;
     const float2 *tcol = p.T + (size_t)slice * H * p.N + i;
     for (int Y = threadIdx.x; Y < H; Y += blockDim.x) {
         const float2 u = tcol[(size_t)Y * p.N], v = two ? tcol[(size_t)Y * p.N + 1] : make_float2(0.f, 0.f);
         const int m = Y ? S - Y : 0;
-        if (m == Y) {   // its own mirror image: real
+        if (!HALF) {
+            sm_bst[Y] = u;
+        } else if (m == Y) {   // its own mirror image: real
             sm_bst[Y] = make_float2(u.x, v.x);
         } else {
             sm_bst[Y] = make_float2(u.x - v.y, u.y + v.x);
@@ -422,21 +433,27 @@ bool bst_plan_shape(BstPlanShape &s, int N, int A, int pad)
     return bst_core_ok(c);
 }
 
-// Polar rows (later the transformed grid rows in their place) and the half grid.
-static size_t bst_polar_bytes(int A, int Lh, int S, int N, int nslices)
+// Polar rows (later the transformed grid rows in their place) and the grid's H rows.
+static size_t bst_polar_bytes(int A, int Lh, int H, int N, int nslices)
 {
-    const size_t polar = (size_t)nslices * 2 * A * Lh, T = (size_t)nslices * (S / 2 + 1) * N;
+    const size_t polar = (size_t)nslices * 2 * A * Lh, T = (size_t)nslices * H * N;
     return (std::max(polar, T) * sizeof(float2) + 255) & ~(size_t)255;
 }
 
-static size_t bst_bytes(int A, int Lh, int S, int N, int nslices)
+static size_t bst_bytes(int A, int Lh, int S, int H, int N, int nslices)
 {
-    return bst_polar_bytes(A, Lh, S, N, nslices) + (size_t)nslices * (S / 2 + 1) * S * sizeof(float2);
+    return bst_polar_bytes(A, Lh, H, N, nslices) + (size_t)nslices * H * S * sizeof(float2);
 }
 
-size_t bst_workspace_bytes(const BstPlanShape &s, int nslices) { return bst_bytes(s.A, s.Lh, s.S, s.N, nslices); }
+size_t bst_workspace_bytes(const BstPlanShape &s, int nslices)
+{
+    return bst_bytes(s.A, s.Lh, s.S, s.S / 2 + 1, s.N, nslices);
+}
 
-size_t bst_core_workspace_bytes(const BstCore &c, int nslices) { return bst_bytes(c.A, c.Lh, c.S, c.N, nslices); }
+size_t bst_core_workspace_bytes(const BstCore &c, int nslices)
+{
+    return bst_bytes(c.A, c.Lh, c.S, c.rows(), c.N, nslices);
+}
 
 // Calls f(integral_constant<int, n>) when n is one of the compiled transform
 // lengths, f(integral_constant<int, 0>) otherwise.
@@ -481,19 +498,22 @@ static void launch_bst_grid(const BstArgs &a, const BstCore &c, int nslices, int
     if (configured != dev) {
         RAFT_CUDA(cudaFuncSetAttribute(bst_gridrows_kernel<NF>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        (int)kBstSmemMax));
-        RAFT_CUDA(cudaFuncSetAttribute(bst_cols_kernel<NF>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        RAFT_CUDA(cudaFuncSetAttribute(bst_cols_kernel<NF, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       (int)kBstSmemMax));
+        RAFT_CUDA(cudaFuncSetAttribute(bst_cols_kernel<NF, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        (int)kBstSmemMax));
         configured = dev;
     }
-    const int H = c.S / 2 + 1;
-    bst_regrid_kernel<<<dim3((c.S + 31) / 32, (H + 7) / 8, (nslices + kRegridSlices - 1) / kRegridSlices), dim3(32, 8), 0,
-                        st>>>(a, nslices);
+    const dim3 grid((c.S + 31) / 32, (a.H + 7) / 8, (nslices + kRegridSlices - 1) / kRegridSlices);
+    if (c.half_grid) bst_regrid_kernel<true><<<grid, dim3(32, 8), 0, st>>>(a, nslices);
+    else bst_regrid_kernel<false><<<grid, dim3(32, 8), 0, st>>>(a, nslices);
     RAFT_CUDA(cudaGetLastError());
     count_launch();
-    bst_gridrows_kernel<NF><<<dim3(H, nslices), threads, sm2, st>>>(a);
+    bst_gridrows_kernel<NF><<<dim3(a.H, nslices), threads, sm2, st>>>(a);
     RAFT_CUDA(cudaGetLastError());
     count_launch();
-    bst_cols_kernel<NF><<<dim3((c.N + 1) / 2, nslices), threads, sm2, st>>>(a);
+    if (c.half_grid) bst_cols_kernel<NF, true><<<dim3((c.N + 1) / 2, nslices), threads, sm2, st>>>(a);
+    else bst_cols_kernel<NF, false><<<dim3(c.N, nslices), threads, sm2, st>>>(a);
     RAFT_CUDA(cudaGetLastError());
 }
 
@@ -507,7 +527,7 @@ void bst_run(int device, const BstCore &c, const float *d_tomo, float *d_obj, in
     a.tomo = d_tomo;
     a.polar = (float2 *)workspace;
     a.T = a.polar;   // the polar rows are read before the grid rows are transformed
-    a.grid = (float2 *)((char *)workspace + bst_polar_bytes(c.A, c.Lh, c.S, c.N, nslices));
+    a.grid = (float2 *)((char *)workspace + bst_polar_bytes(c.A, c.Lh, c.rows(), c.N, nslices));
     a.obj = d_obj;
     a.G = c.G;
     a.pN = c.G ? fft_table(device, c.Np).plan : FftPlan{};
@@ -519,6 +539,7 @@ void bst_run(int device, const BstCore &c, const float *d_tomo, float *d_obj, in
     a.L = c.L;
     a.Lh = c.Lh;
     a.S = c.S;
+    a.H = c.rows();
     a.off = c.off;
     a.M = bst_row_span(c);
     a.w_half = c.w_half;

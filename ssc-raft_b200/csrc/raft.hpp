@@ -294,6 +294,8 @@ struct BstCore {
     bool filtered = false;
     const float2 *G = nullptr;      // filter weights [Np] when filtered
     float w_half = 4.0f, scale = 1.0f;
+    bool half_grid = true;          // transform the grid's Hermitian part (rows 0 .. S/2) only
+    int rows() const { return half_grid ? S / 2 + 1 : S; }
 };
 bool bst_core_ok(const BstCore &c);
 // Compile-time-length transform kernels in use (raft_filter_set_fixed).
