@@ -18,8 +18,10 @@
 // angle-step weight and the output packing for the backprojector all happen
 // in one kernel with the row held in shared memory.  The FFT is a
 // self-sorting (Stockham) mixed-radix transform with radices 2,3,4,5,7,8
-// whose twiddles come from an FP64-built table; lengths with a larger prime
-// factor use a direct circular-convolution kernel instead.  No cuFFT.
+// whose twiddles come from an FP64-built table; rows whose length has a larger
+// prime factor are filtered as a circular convolution inside a longer transform
+// or with Bluestein's algorithm (direct convolution where neither fits shared
+// memory).  No cuFFT.
 #include "raft.hpp"
 #include "profile.hpp"
 #include "fft.cuh"
@@ -27,6 +29,7 @@
 #include <cooperative_groups.h>
 
 #include <cmath>
+#include <complex>
 #include <cstring>
 #include <mutex>
 #include <vector>
@@ -117,6 +120,47 @@ void filter_spectrum_host(int geometry, int ftype, int Np, double paganin, doubl
 }
 
 // ============================================================== host: plan
+// Length (compiled for) of the transform that holds an Np-point circular
+// convolution as a linear one, at least 2 Np - 1; 0: Bluestein's algorithm instead.
+// The convolution takes two transforms per row pair, Bluestein's algorithm four
+// generic ones of that length: 11 x 721 rows of 2002 bins, 688 -> 123 us.  It is
+// also the more accurate one (0.4 - 0.8 of the error against 64 bits), and that is
+// what limits it: Bluestein's error on a filtered row grows with the row's length
+// and with the jump between its ends (1.2e-5 at 2002 bins, 3e-5 at 2039 unpadded
+// ones, 2.6e-5 at 4106), and an image made with it could no longer be reproduced
+// to 1e-5.  So: padded rows of up to 2048 bins, and the nearest-sample operator
+// (linear interpolation doubles the difference).
+static int conv_length(int geometry, int Np, int pad)
+{
+    if (geometry == GEOM_FBP_LIN || pad < 1) return 0;
+    for (int M : {1024, 1536, 2048, 3072, 4096})
+        if (M >= 2 * Np - 1) return M;
+    return 0;
+}
+
+// h[m] = sum_k H[k] exp(2 pi i k m / Np) (real: H is Hermitian) in FP64, by
+// Bluestein's algorithm in a 7-smooth length.
+static std::vector<double> impulse_response(const std::vector<double> &hre, const std::vector<double> &him)
+{
+    using cd = std::complex<double>;
+    const int n = (int)hre.size(), M = fft_plan_length(n);
+    std::vector<cd> w(n), x(M, 0.0), c(M, 0.0), X, C;
+    for (int j = 0; j < n; j++) {
+        const double a = M_PI * (double)(((long long)j * j) % (2LL * n)) / (double)n;
+        w[j] = cd(std::cos(a), std::sin(a));
+        x[j] = cd(hre[j], him[j]) * w[j];
+        c[j] = std::conj(w[j]);
+        if (j) c[M - j] = c[j];
+    }
+    dft_host(x, X);
+    dft_host(c, C);
+    for (int k = 0; k < M; k++) X[k] = std::conj(X[k] * C[k]);
+    dft_host(X, C);   // conj of the unnormalised inverse
+    std::vector<double> h(n);
+    for (int m = 0; m < n; m++) h[m] = (std::conj(C[m]) * w[m]).real() / M;
+    return h;
+}
+
 constexpr size_t kFilterSmemMax = 220 * 1024;
 static int cluster_size_for(int Np, int *radix, int &nradix);
 
@@ -140,17 +184,23 @@ bool build_filter_plan(FilterPlan &plan, int geometry, int ftype, int N, int pad
     const size_t smem = 2 * (size_t)fft_span(Np) * sizeof(float2);   // ping-pong buffers
     plan.fft = factorize(Np, plan.radix, plan.nradix) && smem <= kFilterSmemMax;
     plan.threads = fft_threads(Np);
-    plan.bs_M = 0;
+    plan.conv_M = plan.bs_M = 0;
     if (!plan.fft) {
         // too long for one CTA: a cluster of CTAs, m = Np / C points each
         plan.cluster = cluster_size_for(Np, plan.radix, plan.nradix);
         plan.fft = plan.cluster > 0;
     }
     if (!plan.fft) {
-        // a prime factor above 7: Bluestein's algorithm (two M-point transforms
-        // per direction) when its buffers fit one CTA, else direct convolution
-        const int M = fft_plan_length(Np);
-        if (M > 0 && 2 * (size_t)fft_span(M) * sizeof(float2) <= kFilterSmemMax) {
+        // a prime factor above 7: a convolution inside a longer transform, or
+        // Bluestein's algorithm (two M-point transforms per direction) when its
+        // buffers fit one CTA, else direct convolution
+        const int C = conv_length(geometry, Np, pad), M = fft_plan_length(Np);
+        if (C > 0) {
+            plan.conv_M = C;
+            factorize(C, plan.radix, plan.nradix);
+            plan.threads = fft_threads(C);
+            plan.fft = 1;
+        } else if (M > 0 && 2 * (size_t)fft_span(M) * sizeof(float2) <= kFilterSmemMax) {
             const FftTable &t = fft_table(device, Np);
             plan.bs_M = M;
             plan.bs_chirp = t.plan.chirp;
@@ -163,7 +213,22 @@ bool build_filter_plan(FilterPlan &plan, int geometry, int ftype, int N, int pad
     }
     std::vector<double> hre(Np), him(Np);
     filter_spectrum_host(geometry, ftype, Np, paganin, reg, offset, pixel, hre.data(), him.data());
-    if (plan.fft) {
+    if (plan.conv_M > 0) {
+        // impulse response h = DFT^-1(H) (H carries 1/Np), laid out for lags
+        // -(Np-1) .. Np-1 in M points, transformed in FP64
+        const int M = plan.conv_M;
+        std::vector<std::complex<double>> g(M, 0.0), G;
+        const std::vector<double> h = impulse_response(hre, him);
+        for (int d = 0; d < Np; d++) {
+            g[d] = h[d];
+            if (d) g[M - Np + d] = h[d];
+        }
+        dft_host(g, G);
+        std::vector<float2> H(M);
+        for (int k = 0; k < M; k++) H[k] = make_float2((float)(G[k].real() / M), (float)(G[k].imag() / M));
+        RAFT_CUDA(cudaMalloc(&plan.d_H, sizeof(float2) * M));
+        RAFT_CUDA(cudaMemcpy(plan.d_H, H.data(), sizeof(float2) * M, cudaMemcpyHostToDevice));
+    } else if (plan.fft) {
         std::vector<float2> H(Np), tw(Np);
         for (int k = 0; k < Np; k++) {
             H[k] = make_float2((float)hre[k], (float)him[k]);
@@ -307,18 +372,19 @@ filter_fft_kernel(const float *__restrict__ sino, int N, int Np, int off, int ns
     const bool has1 = rp.a0 + 1 < pk.nangles;
     const float *s0 = sino + (size_t)r0 * N;
     const float *s1 = sino + (size_t)r1 * N;
-    // edge-replicating pad (padding.cu:140-178) of both rows into one complex row
-    for (int n = threadIdx.x; n < Np; n += blockDim.x) {
+    // edge-replicating pad (padding.cu:140-178) of both rows into one complex
+    // row, zero past it (P.n > Np: the transform of a convolution)
+    for (int n = threadIdx.x; n < P.n; n += blockDim.x) {
         int i = n - off;
         i = i < 0 ? 0 : (i > N - 1 ? N - 1 : i);
-        z[n] = make_float2(__ldg(&s0[i]), has1 ? __ldg(&s1[i]) : 0.f);
+        z[n] = n < Np ? make_float2(__ldg(&s0[i]), has1 ? __ldg(&s1[i]) : 0.f) : make_float2(0.f, 0.f);
     }
     __syncthreads();
     if (!skip) {
         z = fft_run(z, zb, P);
         // spectral multiply, then conjugate so that a second forward FFT
         // yields the conjugated inverse transform
-        for (int k = threadIdx.x; k < Np; k += blockDim.x) {
+        for (int k = threadIdx.x; k < P.n; k += blockDim.x) {
             float2 g = cmul(z[k], __ldg(&H[k]));
             z[k] = make_float2(g.x, -g.y);
         }
@@ -351,14 +417,16 @@ filter_fft_kernel(const float *__restrict__ sino, int N, int Np, int off, int ns
 // single-float window rows the last inverse pass stores the window elements
 // from registers (other row formats go through shared memory and pack_row).
 // Bit for bit the results of filter_fft_kernel.
-template <int NP, int R0>
+// CONV: the row's len padded bins are zero-padded to NP points (a convolution).
+template <int NP, int R0, bool CONV>
 struct FxRowsIn {
     const float *s0, *s1;
-    int N, off;
+    int N, off, len;
     bool has1;
     __device__ __forceinline__ float2 operator()(int j, int it, int r) const
     {
         (void)it;
+        if (CONV && j + r * (NP / R0) >= len) return make_float2(0.f, 0.f);
         int i = j + r * (NP / R0) - off;
         i = i < 0 ? 0 : (i > N - 1 ? N - 1 : i);
         return make_float2(__ldg(&s0[i]), has1 ? __ldg(&s1[i]) : 0.f);
@@ -388,11 +456,11 @@ struct FxSpecLast {
 struct FxWindow {
     float *out;
     size_t base0, base1;   // element 0 of the two window rows
-    int stride, wlo, Wg;
+    int stride, wlo, Wg, len;
     float w0, w1;
     bool has1;
 };
-template <int R, int NS>
+template <int R, int NS, bool CONV>
 struct FxWinOut {
     FxWindow w;
     __device__ __forceinline__ void operator()(int q, int k, const float2 (&v)[R]) const
@@ -402,15 +470,16 @@ struct FxWinOut {
         for (int r = 0; r < R; r++) {
             const int e = k + r * NS - w.wlo;
             if ((unsigned)e < (unsigned)w.Wg) {
-                w.out[w.base0 + (size_t)e * w.stride] = v[r].x * w.w0;
-                if (w.has1) w.out[w.base1 + (size_t)e * w.stride] = (-v[r].y) * w.w1;
+                const bool in = !CONV || k + r * NS < w.len;   // points past the row are not its bins
+                w.out[w.base0 + (size_t)e * w.stride] = in ? v[r].x * w.w0 : 0.f;
+                if (w.has1) w.out[w.base1 + (size_t)e * w.stride] = in ? (-v[r].y) * w.w1 : 0.f;
             }
         }
     }
 };
-struct FxWinLast {
+template <bool CONV> struct FxWinLast {
     FxWindow w;
-    template <int R, int NS> __device__ __forceinline__ FxWinOut<R, NS> at() const { return {w}; }
+    template <int R, int NS> __device__ __forceinline__ FxWinOut<R, NS, CONV> at() const { return {w}; }
 };
 
 // CTAs per SM the launch bounds ask for: as many as shared memory and the
@@ -425,10 +494,10 @@ __host__ __device__ constexpr int fixed_filter_min_blocks(int NP)
                       65536 / (64 * c_fft_threads(NP)));
 }
 
-template <int NP, bool IL, bool FUSED>
+template <int NP, bool IL, bool FUSED, bool CONV>
 __global__ void __launch_bounds__(c_fft_threads(NP), fixed_filter_min_blocks(NP))
-filter_fixed_kernel(const float *__restrict__ sino, int N, int off, int nslices, const float2 *__restrict__ H,
-                    PackArgs pk)
+filter_fixed_kernel(const float *__restrict__ sino, int N, int len, int off, int nslices,
+                    const float2 *__restrict__ H, PackArgs pk)
 {
     constexpr CRadices rl = c_factorize(NP);
     constexpr int T = c_fft_threads(NP);
@@ -442,7 +511,7 @@ filter_fixed_kernel(const float *__restrict__ sino, int N, int off, int nslices,
     const int r0 = rp.k * pk.nangles + rp.a0, r1 = r0 + 1;
     const bool has1 = rp.a0 + 1 < pk.nangles;
     // forward transform of the two edge-padded rows, times H, conjugated
-    const FxRowsIn<NP, rl.r[0]> rows{sino + (size_t)r0 * N, sino + (size_t)r1 * N, N, off, has1};
+    const FxRowsIn<NP, rl.r[0], CONV> rows{sino + (size_t)r0 * N, sino + (size_t)r1 * N, N, off, len, has1};
     float2 *X = cfft_out_buffer<NP>() ? B : A, *Y = (X == A) ? B : A;
     cfft_passes<NP, 0, 1>(A, B, rows, FxSpecLast{X, H});
     __syncthreads();
@@ -457,10 +526,11 @@ filter_fixed_kernel(const float *__restrict__ sino, int N, int off, int nslices,
         w.base1 = w.base0 + (size_t)pk.Wg * w.stride;
         w.wlo = pk.wlo;
         w.Wg = pk.Wg;
+        w.len = len;
         w.w0 = pk.wt ? pk.wt[rp.a0] : 1.f;
         w.w1 = (pk.wt && has1) ? pk.wt[rp.a0 + 1] : 1.f;
         w.has1 = has1;
-        cfft_passes<NP, 0, 1>(X, Y, spec, FxWinLast{w});
+        cfft_passes<NP, 0, 1>(X, Y, spec, FxWinLast<CONV>{w});
         // window elements outside the padded row
         const int lo = min(pk.Wg, max(0, -pk.wlo)), hi = max(0, NP - pk.wlo);
         for (int e = threadIdx.x; e < pk.Wg; e += T) {
@@ -480,7 +550,7 @@ filter_fixed_kernel(const float *__restrict__ sino, int N, int off, int nslices,
 static bool g_fixed_filter = true;
 bool fixed_transforms_enabled() { return g_fixed_filter; }
 
-template <int NP, bool IL, bool FUSED>
+template <int NP, bool IL, bool FUSED, bool CONV>
 static void launch_fixed_one(const FilterPlan &plan, const FilterLaunch &fl, const PackArgs &pk, int nsl,
                              cudaStream_t st)
 {
@@ -489,45 +559,58 @@ static void launch_fixed_one(const FilterPlan &plan, const FilterLaunch &fl, con
     cudaGetDevice(&dev);
     const size_t smem = 2 * (size_t)fft_span(NP) * sizeof(float2);
     if (configured_dev != dev) {
-        RAFT_CUDA(cudaFuncSetAttribute(filter_fixed_kernel<NP, IL, FUSED>,
+        RAFT_CUDA(cudaFuncSetAttribute(filter_fixed_kernel<NP, IL, FUSED, CONV>,
                                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        RAFT_CUDA(cudaFuncSetAttribute(filter_fixed_kernel<NP, IL, FUSED>,
+        RAFT_CUDA(cudaFuncSetAttribute(filter_fixed_kernel<NP, IL, FUSED, CONV>,
                                        cudaFuncAttributePreferredSharedMemoryCarveout, 100));
         configured_dev = dev;
     }
     ProfScope ps(PROF_FILTER, st);
-    filter_fixed_kernel<NP, IL, FUSED><<<(unsigned)row_pairs(nsl, fl.nangles, IL), c_fft_threads(NP), smem, st>>>(
-        fl.sino, plan.N, plan.off, nsl, plan.d_H, pk);
+    filter_fixed_kernel<NP, IL, FUSED, CONV><<<(unsigned)row_pairs(nsl, fl.nangles, IL), c_fft_threads(NP), smem, st>>>(
+        fl.sino, plan.N, plan.Np, plan.off, nsl, plan.d_H, pk);
 }
 
-template <int NP>
+template <int NP, bool CONV>
 static void launch_fixed_np(const FilterPlan &plan, const FilterLaunch &fl, const PackArgs &pk, int nsl,
                             cudaStream_t st)
 {
     const bool f32 = fl.store == STORE_F32;
     if (fl.interleaved) {
-        if (f32) launch_fixed_one<NP, true, true>(plan, fl, pk, nsl, st);
-        else launch_fixed_one<NP, true, false>(plan, fl, pk, nsl, st);
+        if (f32) launch_fixed_one<NP, true, true, CONV>(plan, fl, pk, nsl, st);
+        else launch_fixed_one<NP, true, false, CONV>(plan, fl, pk, nsl, st);
     } else {
-        if (f32) launch_fixed_one<NP, false, true>(plan, fl, pk, nsl, st);
-        else launch_fixed_one<NP, false, false>(plan, fl, pk, nsl, st);
+        if (f32) launch_fixed_one<NP, false, true, CONV>(plan, fl, pk, nsl, st);
+        else launch_fixed_one<NP, false, false, CONV>(plan, fl, pk, nsl, st);
     }
 }
 
-// Runs the fixed-length filter when one is compiled for plan.Np.
+template <int NP>
+static void launch_fixed_len(const FilterPlan &plan, const FilterLaunch &fl, const PackArgs &pk, int nsl,
+                            cudaStream_t st)
+{
+    if constexpr (NP <= 4096) {   // conv_length
+        if (plan.conv_M > 0) {
+            launch_fixed_np<NP, true>(plan, fl, pk, nsl, st);
+            return;
+        }
+    }
+    launch_fixed_np<NP, false>(plan, fl, pk, nsl, st);
+}
+
+// Runs the fixed-length filter when one is compiled for the transform length.
 static bool launch_fixed_filter(const FilterPlan &plan, const FilterLaunch &fl, const PackArgs &pk, int nsl,
                                 cudaStream_t st)
 {
     if (!g_fixed_filter) return false;
-    switch (plan.Np) {
-    case 1024: launch_fixed_np<1024>(plan, fl, pk, nsl, st); return true;
-    case 1536: launch_fixed_np<1536>(plan, fl, pk, nsl, st); return true;
-    case 2048: launch_fixed_np<2048>(plan, fl, pk, nsl, st); return true;
-    case 3072: launch_fixed_np<3072>(plan, fl, pk, nsl, st); return true;
-    case 4096: launch_fixed_np<4096>(plan, fl, pk, nsl, st); return true;
-    case 6144: launch_fixed_np<6144>(plan, fl, pk, nsl, st); return true;
-    case 8192: launch_fixed_np<8192>(plan, fl, pk, nsl, st); return true;
-    case 12288: launch_fixed_np<12288>(plan, fl, pk, nsl, st); return true;
+    switch (plan.conv_M > 0 ? plan.conv_M : plan.Np) {
+    case 1024: launch_fixed_len<1024>(plan, fl, pk, nsl, st); return true;
+    case 1536: launch_fixed_len<1536>(plan, fl, pk, nsl, st); return true;
+    case 2048: launch_fixed_len<2048>(plan, fl, pk, nsl, st); return true;
+    case 3072: launch_fixed_len<3072>(plan, fl, pk, nsl, st); return true;
+    case 4096: launch_fixed_len<4096>(plan, fl, pk, nsl, st); return true;
+    case 6144: launch_fixed_len<6144>(plan, fl, pk, nsl, st); return true;
+    case 8192: launch_fixed_len<8192>(plan, fl, pk, nsl, st); return true;
+    case 12288: launch_fixed_len<12288>(plan, fl, pk, nsl, st); return true;
     default: return false;
     }
 }
@@ -811,8 +894,8 @@ void launch_filter(const FilterPlan &plan, const FilterLaunch &fl, cudaStream_t 
     }
     if (plan.fft || plan.skip) {
         FftPlan P;
-        P.n = plan.Np;
-        P.M = plan.bs_M > 0 ? plan.bs_M : plan.Np;
+        P.n = plan.conv_M > 0 ? plan.conv_M : plan.Np;
+        P.M = plan.bs_M > 0 ? plan.bs_M : P.n;
         P.rl.n = plan.skip ? 0 : plan.nradix;
         for (int i = 0; i < P.rl.n; i++) P.rl.r[i] = plan.radix[i];
         P.chirp = plan.bs_chirp;

@@ -80,12 +80,13 @@ struct FilterPlan {
     int N = 0, Np = 0, pad = 0, off = 0;
     int fft = 0;                 // 1: mixed-radix FFT path, 0: direct circular convolution
     int cluster = 0;             // > 1: FFT by a cluster of this many CTAs (radix = of Np / cluster)
+    int conv_M = 0;              // > 0: circular convolution inside a transform of this length (radix, d_H of it)
     int bs_M = 0;                // > 0: Bluestein transforms of this length (radix = of bs_M)
     const float2 *bs_chirp = nullptr, *bs_B = nullptr;   // Bluestein tables (cached per device and length)
     int nradix = 0;
     int radix[24] = {};
     int threads = 0;             // CTA size of the FFT kernel
-    float2 *d_H = nullptr;       // full Hermitian-extended spectrum incl. 1/(Np*pixel)
+    float2 *d_H = nullptr;       // full Hermitian-extended spectrum incl. 1/(Np*pixel) (1/conv_M in its place)
     float2 *d_tw = nullptr;      // exp(-2 pi i m / Np)
     float *d_h = nullptr;        // impulse response (direct path)
     bool skip = false;           // reference 'none' filter: pad + copy only
