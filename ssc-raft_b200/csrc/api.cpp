@@ -360,7 +360,7 @@ int raft_fbp_device(int gpu, float *d_obj, const float *d_tomogram, const float 
         RAFT_CUDA(cudaSetDevice(gpu));
         ds.ensure();
         cudaStream_t st = resolve_stream(ds, stream, ds.s_comp);
-        FbpPrepared fp = prepare_fbp(cfg, gpu);
+        FbpPrepared fp = prepare_fbp(cfg, gpu, angles);
         FbpTables tb = fbp_tables(ds, fp, angles, st);
         const size_t tomo_ps = (size_t)cfg.nangles * cfg.nrays;
         const int chunk = std::max(1, std::min(cfg.nslices, cfg.blocksize > 0 ? cfg.blocksize : 32));

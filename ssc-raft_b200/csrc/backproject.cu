@@ -36,6 +36,7 @@
 #include <mutex>
 #include <string>
 #include <tuple>
+#include <type_traits>
 #include <vector>
 
 namespace raft {
@@ -63,6 +64,7 @@ struct BpArgs {
     int *err;
     int update;                  // 0: store, 1: img = img * acc / den
     int il;                      // 1: filt holds groups of 4 slices interleaved, [group][angle][Wg][4 elements]
+    float eps;                   // run kernel: bound on the rounding of a bin position (bins)
 };
 
 constexpr uint32_t kWaitLimit = 1u << 24;
@@ -74,15 +76,17 @@ static_assert(kWinOffset % 128 == 0, "window area alignment");
 // ------------------------------------------------------------------------
 // per-angle window base (warp 0, one lane per angle)
 // ------------------------------------------------------------------------
-template <int GEOM>
-__device__ __forceinline__ void angle_param(const BpArgs &p, int a, int x0, int y0, AngleParam &ap, int &base)
+// tmin_i: lowest padded-bin index of the tile's corners (nearest-sample geometries)
+template <int GEOM, int TX, int TY>
+__device__ __forceinline__ void angle_param(const BpArgs &p, int a, int x0, int y0, AngleParam &ap, int &base,
+                                            int &tmin_i)
 {
     const int align = 16 / p.esize;
     int lo;
     if constexpr (GEOM == GEOM_FBP_LIN) {
         const double c = p.csd[a], s = -p.snd[a] * p.ratio;
         const double v00 = ((double)x0 + p.c0) * c + ((double)y0 + p.c0) * s + p.u0;
-        const double vmin = v00 + fmin(0.0, (BP_TX - 1) * c) + fmin(0.0, (BP_TY - 1) * s);
+        const double vmin = v00 + fmin(0.0, (TX - 1) * c) + fmin(0.0, (TY - 1) * s);
         lo = (int)floor(vmin) - 1;
         int b = lo - ((lo % align) + align) % align;
         b = max(0, min(b, p.Wg - p.W));
@@ -93,12 +97,12 @@ __device__ __forceinline__ void angle_param(const BpArgs &p, int a, int x0, int 
         ap.d = b;
     } else {
         const float c = p.cs[a], s = p.sn[a];
-        int tmin_i = 0x7fffffff;
+        tmin_i = 0x7fffffff;
 #pragma unroll
         for (int cy = 0; cy < 2; cy++)
 #pragma unroll
             for (int cx = 0; cx < 2; cx++) {
-                const int i = x0 + cx * (BP_TX - 1), j = y0 + cy * (BP_TY - 1);
+                const int i = x0 + cx * (TX - 1), j = y0 + cy * (TY - 1);
                 int ti;
                 // the corner bins need not match bp_tile's per-pixel rounding
                 // exactly: the window starts one bin below the lowest corner
@@ -151,7 +155,7 @@ __device__ __forceinline__ float lerp_fetch(const unsigned char *w, int k, float
 // are computed once per (pixel, angle) and reused for every slice, whose
 // windows sit side by side in shared memory ([angle][slice][W]).  With IL
 // (S = 4) the rows arrive interleaved by slice ([group][angle][Wg][4
-// elements], see interleave4_kernel), the staged windows are [angle][W][4]
+// elements]), the staged windows are [angle][W][4]
 // and one 16-byte load (two for f32 pairs) fetches the sample of all four
 // slices: one bulk copy per angle instead of four, one or two shared-memory
 // instructions per (pixel, angle) instead of four.  AB (angles per pipeline stage) is a launch
@@ -197,8 +201,8 @@ __device__ __forceinline__ bool bp_tile(const BpArgs &p, const int AB, const int
         const int na = min(AB, A - a0);
         if (lane < na) {
             AngleParam ap;
-            int base;
-            angle_param<GEOM>(p, a0 + lane, x0, y0, ap, base);
+            int base, tmin_i;
+            angle_param<GEOM, BP_TX, BP_TY>(p, a0 + lane, x0, y0, ap, base, tmin_i);
             prm[b * 32 + lane] = ap;
         }
         if (lane == 0) {
@@ -410,24 +414,11 @@ __global__ void __launch_bounds__(BP_THREADS, 3) bp_kernel_s4(const BpArgs p, co
     bp_body<GEOM, STORE, 4, IL>(p, AB);
 }
 
-// Window rows [nslices][nangles][Wg] of 4-byte (E = uint32_t: f32, bf16 pair) or
-// 8-byte (E = uint2: f32 pair) elements -> [ceil(nslices/4)][nangles][Wg][4],
-// slices beyond nslices zero; a bit copy, one CTA per (group, angle) row.
-template <typename E>
-__global__ void interleave4_kernel(const E *__restrict__ rows, E *__restrict__ out, int nslices, int A, int Wg)
-{
-    const int r = blockIdx.x, g = r / A, a = r - g * A;
-    const E *src[4];
-#pragma unroll
-    for (int q = 0; q < 4; q++) src[q] = 4 * g + q < nslices ? rows + ((size_t)(4 * g + q) * A + a) * Wg : nullptr;
-    E *dst = out + (size_t)r * Wg * 4;
-    E zero;
-    memset(&zero, 0, sizeof(E));
-    for (int e = threadIdx.x; e < Wg; e += blockDim.x) {
-#pragma unroll
-        for (int q = 0; q < 4; q++) dst[4 * e + q] = src[q] ? __ldcs(src[q] + e) : zero;
-    }
-}
+}  // namespace raft
+
+#include "bp_run.cuh"
+
+namespace raft {
 
 // ------------------------------------------------------------------------
 // Ragged persistent backprojector: many requests (different image sizes,
@@ -595,6 +586,11 @@ WindowLayout plan_window(const BpPlanInput &in)
     // staged window: tile span, +1 inclusive, 1 bin margin each side,
     // rounding of the aligned start, 1 extra for the lin pair index rounding
     L.W = ceil_to((int)std::ceil(span) + 1 + 2 + (align - 1) + 2, align);
+    // run kernel: one bin below the lowest corner, rounded down to `align` (as the
+    // other kernels round, so that linear positions are the same floats), the span
+    // and its roundings, up to four elements past the last bin
+    const double bin = in.geometry == GEOM_EM_REF ? in.dxy / in.dt : std::max(in.dx, in.dy) / in.dt;
+    L.Wrun = (int)std::ceil(bin * std::hypot(31.0, 31.0)) + 8 + align;
     L.wlo = floor_to((int)std::floor(lo) - 4 - align, align);
     const int whi = (int)std::ceil(hi) + 4 + L.W + align;
     L.Wg = ceil_to(whi - L.wlo, align);
@@ -631,6 +627,116 @@ static void launch_bp_s(const BpArgs &a, int AB, cudaStream_t st)
     ProfScope ps(PROF_BACKPROJECT, st);
     kern<<<grid, BP_THREADS, smem, st>>>(a, AB);
     RAFT_CUDA(cudaGetLastError());
+}
+
+struct BpTune;
+static bool forced_tune(BpTune &t);
+
+// The run kernel: its rule on positions needs pixels as wide as detector bins.
+// Turning the accumulators costs about as much as three angles, so angle lists
+// that change the run axis more often than every 16 angles (scans in
+// golden-ratio order) keep the single-pixel kernel.
+bool bp_runs_ok(const BpGeo &g, int geometry, int nangles, int turns)
+{
+    if (turns > nangles / 16 + 2) return false;
+    if (geometry == GEOM_EM_REF) return g.dxy == g.dt;
+    return g.dx == g.dt && g.dy == g.dt && g.ratio == 1.0;
+}
+
+// A single slice of four-byte elements: plain rows and the one-slice form of the
+// run kernel (512^2 x 360: 50 us; 102 us when it filled a quarter of a four-slice
+// CTA).  Two and three slices of a small image are no faster as one-slice CTAs
+// (3 x 301^2 x 257: 53 us against 50 us).
+bool bp_run_plain(const BpGeo &g, int geometry, int store, int nslices, int nangles, int turns)
+{
+    BpTune forced;
+    return nslices == 1 && store_bytes(store) == 4 && bp_runs_ok(g, geometry, nangles, turns) && !forced_tune(forced);
+}
+
+int bp_run_turns(const float *angles, int nangles)
+{
+    int turns = 0;
+    bool last = false;
+    for (int a = 0; a < nangles; a++) {
+        const bool along_y = std::fabs(std::cos(angles[a])) > std::fabs(std::sin(angles[a]));
+        if (a > 0 && along_y != last) turns++;
+        last = along_y;
+    }
+    return turns;
+}
+
+template <int GEOM, int STORE, bool UNIT, int G>
+static void launch_run_t(BpArgs a, int AB, int group0, int groups, cudaStream_t st)
+{
+    const size_t smem = kRunFixed + kRunStages * (size_t)AB * a.W * (G ? 16 * G : 4);
+    RAFT_CHECK(smem <= kBpSmemMax && AB >= 1 && AB <= 32, "backprojector: staged window too large");
+    static thread_local int configured = -1;
+    int dev = 0;
+    cudaGetDevice(&dev);
+    auto kern = bp_run_kernel<GEOM, STORE, UNIT, G>;
+    if (configured != dev) {
+        RAFT_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kBpSmemMax));
+        configured = dev;
+    }
+    a.filt += (size_t)group0 * a.nangles * a.Wg * 16;
+    a.img += (size_t)group0 * 4 * a.No * a.No;
+    if (a.den) a.den += (size_t)group0 * 4 * a.No * a.No;
+    a.nslices -= 4 * group0;
+    dim3 grid((a.No + kRunTile - 1) / kRunTile, (a.No + kRunTile - 1) / kRunTile, groups / (G ? G : 1));
+    ProfScope ps(PROF_BACKPROJECT, st);
+    kern<<<grid, BP_THREADS, smem, st>>>(a, AB);
+    RAFT_CUDA(cudaGetLastError());
+}
+
+template <int GEOM, int STORE, bool UNIT>
+static void launch_run_s(BpArgs a, const WindowLayout &win, cudaStream_t st)
+{
+    if (!a.il) {   // one slice per CTA on plain rows
+        if constexpr (STORE != STORE_PAIR_F32) {
+            a.W = (win.Wrun + 3) & ~3;
+            launch_run_t<GEOM, STORE, UNIT, 0>(a, 32, 0, a.nslices, st);
+        }
+        return;
+    }
+    // Sixteen or eight slices per thread share a position's arithmetic where that
+    // leaves every SM the two CTAs that fit it; else, and for what is left over,
+    // four.  32 x 2048^2 x 1800, nearest: 25.2, 26.2 and 31.5 ms per pass (the
+    // single-pixel kernel 31.5); linear interpolation, whose bins take twice the
+    // registers, gains nothing from sixteen (11.05 ms either way).
+    const int groups = (a.nslices + 3) / 4;
+    const long long tiles = (long long)((a.No + kRunTile - 1) / kRunTile) * ((a.No + kRunTile - 1) / kRunTile);
+    a.W = win.Wrun;
+    int g0 = 0;
+    if constexpr (STORE == STORE_F32) {
+        const int n = groups / 4;
+        if (tiles * n >= 2 * 148) {
+            launch_run_t<GEOM, STORE, UNIT, 4>(a, 8, 0, 4 * n, st);
+            g0 = 4 * n;
+        }
+    }
+    if (const int n = (groups - g0) / 2; tiles * n >= 2 * 148) {
+        launch_run_t<GEOM, STORE, UNIT, 2>(a, 16, g0, 2 * n, st);
+        g0 += 2 * n;
+    }
+    if (g0 < groups) launch_run_t<GEOM, STORE, UNIT, 1>(a, 16, g0, groups - g0, st);
+}
+
+static void launch_run(BpArgs a, const WindowLayout &win, int geometry, int store, cudaStream_t st)
+{
+    const double umax = std::max(std::abs(win.wlo), std::abs(win.wlo + win.Wg));
+    a.eps = 1e-3f + (geometry == GEOM_FBP_LIN ? 0.f : (float)(umax / (1 << 20)));
+    switch (geometry) {
+    case GEOM_FBP_REF:
+        // bins of unit width (pixel size 1, the default): no multiplication by 1 / dt
+        if (a.dt == 1.f) launch_run_s<GEOM_FBP_REF, STORE_F32, true>(a, win, st);
+        else launch_run_s<GEOM_FBP_REF, STORE_F32, false>(a, win, st);
+        break;
+    case GEOM_EM_REF: launch_run_s<GEOM_EM_REF, STORE_F32, false>(a, win, st); break;
+    default:
+        if (store == STORE_PAIR_BF16) launch_run_s<GEOM_FBP_LIN, STORE_PAIR_BF16, true>(a, win, st);
+        else launch_run_s<GEOM_FBP_LIN, STORE_PAIR_F32, true>(a, win, st);
+        break;
+    }
 }
 
 template <int GEOM, int STORE>
@@ -694,17 +800,13 @@ bool bp_forced_planar()
 
 // Pick (S, AB) for this configuration: the cached choice, else time every
 // candidate that fits shared memory on 8 to 32 slices of the real data
-// (store launches only -- they are idempotent), else a default.  With
-// a_il (the same launch on slice-interleaved rows) the S = 4 candidates are
-// timed on it; prep_il makes those rows and is called at most once.  With
-// il_only the rows exist only interleaved: the S = 4 candidates alone.
-template <class Prep>
-static BpTune choose_tune(const BpArgs &a, const BpArgs *a_il, Prep &&prep_il, int geometry, int store,
-                          cudaStream_t st, bool il_only = false)
+// (store launches only -- they are idempotent), else a default.  With il_only
+// the rows are interleaved by slice: the S = 4 candidates alone.
+static BpTune choose_tune(const BpArgs &a, int geometry, int store, cudaStream_t st, bool il_only = false)
 {
     int dev = 0;
     cudaGetDevice(&dev);
-    const TuneKey key(dev, geometry, store + (a_il ? 16 : 0) + (il_only ? 32 : 0), a.No, a.W, a.nangles);
+    const TuneKey key(dev, geometry, store + (il_only ? 32 : 0), a.No, a.W, a.nangles);
     const int esize = store_bytes(store);
     BpTune forced;
     if (forced_tune(forced) && bp_smem(forced.S, forced.AB, a.W, esize) <= kBpSmemMax && (!il_only || forced.S == 4))
@@ -739,18 +841,12 @@ static BpTune choose_tune(const BpArgs &a, const BpArgs *a_il, Prep &&prep_il, i
         for (const BpTune &c : kTuneCandidates) {
             if (bp_smem(c.S, c.AB, a.W, esize) > kBpSmemMax) continue;
             if (il_only && c.S != 4) continue;
-            BpArgs t = t0;
-            if (c.S == 4 && a_il) {
-                prep_il();
-                t = *a_il;
-                t.nslices = t0.nslices;
-            }
-            launch_bp_any(t, geometry, store, c, st);   // warm
+            launch_bp_any(t0, geometry, store, c, st);   // warm
             // the fastest of three single launches (less sensitive to a stray slow one)
             float ms = 1e30f;
             for (int rep = 0; rep < 3; rep++) {
                 RAFT_CUDA(cudaEventRecord(e0, st));
-                launch_bp_any(t, geometry, store, c, st);
+                launch_bp_any(t0, geometry, store, c, st);
                 RAFT_CUDA(cudaEventRecord(e1, st));
                 RAFT_CUDA(cudaEventSynchronize(e1));
                 float one = 0.f;
@@ -831,44 +927,24 @@ void launch_backproject(const BpLaunch &bl, cudaStream_t st)
     if (bl.nslices <= 0 || bl.nangles <= 0) return;
     const BpArgs a = to_args(bl);
     const int store = bl.geometry == GEOM_FBP_LIN ? bl.store : STORE_F32;
-    // four slices per CTA on slice-interleaved rows, when the caller provides the workspace
-    // (4-byte elements: f32 samples and bf16 pairs; the 8-byte f32 pairs keep
-    // their planar rows, whose S = 4 shape measured faster)
-    const bool il_ok = bl.il_ws != nullptr && a.esize == 4;
-    BpArgs a_il = a;
-    a_il.filt = reinterpret_cast<const unsigned char *>(bl.il_ws);
-    a_il.il = 1;
     if (bl.il_ready) {
-        // the filter wrote the rows interleaved: four slices per CTA only
-        RAFT_CHECK(il_ok, "backprojector: interleaved rows need the workspace and 4-byte elements");
-        auto none = []() {};
-        const BpTune t = choose_tune(a_il, &a_il, none, bl.geometry, store, st, true);
-        launch_bp_any(a_il, bl.geometry, store, t, st);
+        // rows interleaved by slice in groups of four
+        BpArgs a_il = a;
+        a_il.filt = reinterpret_cast<const unsigned char *>(bl.il_ws);
+        a_il.il = 1;
+        if (bp_runs_ok(bl.geo, bl.geometry, bl.nangles, bl.turns)) {
+            launch_run(a_il, bl.win, bl.geometry, store, st);
+            return;
+        }
+        RAFT_CHECK(a.esize == 4, "backprojector: interleaved rows need 4-byte elements");
+        launch_bp_any(a_il, bl.geometry, store, choose_tune(a_il, bl.geometry, store, st, true), st);
         return;
     }
-    bool il_done = false;
-    auto prep_il = [&]() {
-        if (il_done) return;
-        count_launch();
-        const unsigned grid = (unsigned)(((bl.nslices + 3) / 4) * bl.nangles);
-        if (a.esize == 8)
-            interleave4_kernel<uint2><<<grid, 256, 0, st>>>(reinterpret_cast<const uint2 *>(bl.filt),
-                                                          reinterpret_cast<uint2 *>(bl.il_ws), bl.nslices,
-                                                          bl.nangles, bl.win.Wg);
-        else
-            interleave4_kernel<uint32_t><<<grid, 256, 0, st>>>(reinterpret_cast<const uint32_t *>(bl.filt),
-                                                             reinterpret_cast<uint32_t *>(bl.il_ws), bl.nslices,
-                                                             bl.nangles, bl.win.Wg);
-        RAFT_CUDA(cudaGetLastError());
-        il_done = true;
-    };
-    const BpTune t = choose_tune(a, il_ok ? &a_il : nullptr, prep_il, bl.geometry, store, st);
-    if (il_ok && t.S == 4) {
-        prep_il();
-        launch_bp_any(a_il, bl.geometry, store, t, st);
-    } else {
-        launch_bp_any(a, bl.geometry, store, t, st);
+    if (bp_run_plain(bl.geo, bl.geometry, store, bl.nslices, bl.nangles, bl.turns)) {
+        launch_run(a, bl.win, bl.geometry, store, st);
+        return;
     }
+    launch_bp_any(a, bl.geometry, store, choose_tune(a, bl.geometry, store, st), st);
 }
 
 // ------------------------------------------------------------------------

@@ -266,7 +266,7 @@ static int auto_chunk(int nslices, size_t bytes_per_slice, int blocksize)
 }
 
 // ------------------------------------------------------------------ FBP --
-FbpPrepared prepare_fbp(const FbpConfig &cfg, int device)
+FbpPrepared prepare_fbp(const FbpConfig &cfg, int device, const float *h_angles)
 {
     FbpPrepared fp;
     fp.cfg = cfg;
@@ -300,6 +300,7 @@ FbpPrepared prepare_fbp(const FbpConfig &cfg, int device)
     g.u0 = 0.5 * fp.Np - fp.win.wlo - 0.5;
     fp.plan = &cached_filter_plan(device, cfg.geometry, cfg.filter, N, pad, cfg.paganin, cfg.reg, cfg.offset,
                                   cfg.pixel_x);
+    if (h_angles) fp.turns = bp_run_turns(h_angles, cfg.nangles);
     return fp;
 }
 
@@ -346,7 +347,9 @@ void fbp_chunk(DeviceState &ds, const FbpPrepared &fp, const FbpTables &tb, cons
     if (nslices <= 0) return;
     // with the interleave workspace and 4-byte elements the filter writes the
     // four-slice interleaved rows the backprojector stages, directly
-    const bool fused = d_il && fbp_fused_il(fp);
+    const bool plain = d_il && bp_run_plain(fp.geo, fp.cfg.geometry, fp.cfg.store, nslices, fp.cfg.nangles, fp.turns);
+    const bool fused = d_il && !plain && fbp_fused_il(fp);
+    if (plain) d_rows = d_il;   // plain rows in the interleaved ones' place
     FilterLaunch fl;
     fl.sino = d_sino;
     fl.out = fused ? d_il : d_rows;
@@ -356,7 +359,9 @@ void fbp_chunk(DeviceState &ds, const FbpPrepared &fp, const FbpTables &tb, cons
     fl.nangles = fp.cfg.nangles;
     fl.wlo = fp.win.wlo;
     fl.Wg = fp.win.Wg;
-    fl.store = fp.cfg.store;
+    // linear interpolation in FP32: interleaved rows hold single floats (the run
+    // kernel forms the pairs), planar ones pairs
+    fl.store = fused && fp.cfg.store == STORE_PAIR_F32 ? (int)STORE_F32 : fp.cfg.store;
     launch_filter(*fp.plan, fl, st);
     BpLaunch bl;
     bl.filt = fused ? nullptr : d_rows;
@@ -375,12 +380,15 @@ void fbp_chunk(DeviceState &ds, const FbpPrepared &fp, const FbpTables &tb, cons
     bl.err = tb.err;
     bl.il_ws = d_il;
     bl.il_ready = fused ? 1 : 0;
+    bl.turns = fp.turns;
     launch_backproject(bl, st);
 }
 
 size_t fbp_il_bytes(const FbpPrepared &fp, int nslices)
 {
-    return store_bytes(fp.cfg.store) == 4 ? bp_il_bytes(nslices, fp.cfg.nangles, fp.win.Wg, 4) : 0;
+    // pairs of floats are read by the run kernel only (from single floats)
+    const bool il = store_bytes(fp.cfg.store) == 4 || bp_runs_ok(fp.geo, fp.cfg.geometry, fp.cfg.nangles, fp.turns);
+    return il ? bp_il_bytes(nslices, fp.cfg.nangles, fp.win.Wg, 4) : 0;
 }
 
 static void check_device_flag(const int *d_err, const char *what)
@@ -398,7 +406,7 @@ void fbp_host_slab(const FbpConfig &cfg, int device, float *obj, const float *to
     std::lock_guard<std::mutex> lk(ds.mtx);
     RAFT_CUDA(cudaSetDevice(device));
     ds.ensure();
-    FbpPrepared fp = prepare_fbp(cfg, device);
+    FbpPrepared fp = prepare_fbp(cfg, device, angles);
     FbpTables tb = fbp_tables(ds, fp, angles, ds.s_comp);
     const size_t in_ps = (size_t)cfg.nangles * cfg.nrays * sizeof(float);
     const size_t out_ps = (size_t)fp.No * fp.No * sizeof(float);
@@ -676,13 +684,15 @@ void em_chunk(DeviceState &ds, const EmPrepared &ep, int kind, const float *d_da
     launch_angle_tables(d_ang, A, cs, sn, wt, 1, st);
 
     const WindowLayout &win = ep.win;
-    const size_t rows_bytes = (size_t)nslices * A * win.Wg * sizeof(float);
-    float *rows = (float *)ds.rows.get(rows_bytes);
+    // window rows interleaved by slice, as the four-slice backprojector stages
+    // them: written by to_window4 (sensitivity image) and the projector
+    // (iterations); margins and slices past the batch stay zero from this clear
+    const size_t rows_bytes = bp_il_bytes(nslices, A, win.Wg, 4);
+    float *rows = (float *)ds.il.get(rows_bytes);
     RAFT_CUDA(cudaMemsetAsync(rows, 0, rows_bytes, st));
     float *den = (float *)ds.den.get((size_t)nslices * N * N * sizeof(float));
 
     BpLaunch bl;
-    bl.filt = rows;
     bl.No = N;
     bl.nangles = A;
     bl.nslices = nslices;
@@ -693,10 +703,20 @@ void em_chunk(DeviceState &ds, const EmPrepared &ep, int kind, const float *d_da
     bl.cs = cs;
     bl.sn = sn;
     bl.err = err;
-    bl.il_ws = ds.il.get(bp_il_bytes(nslices, A, win.Wg, 4));
+    bl.turns = bp_run_turns(h_angles, A);
+    // one slice: plain rows
+    const bool plain = bp_run_plain(ep.geo, GEOM_EM_REF, STORE_F32, nslices, A, bl.turns);
+    if (plain) {
+        bl.filt = rows;
+    } else {
+        bl.il_ws = rows;
+        bl.il_ready = 1;
+    }
 
     // sensitivity image: BP of the counts (tEM, em_rt.cu:178) or of ones (eEM, :343)
-    launch_to_window(kind == 0 ? d_data : nullptr, rows, wt, nslices * A, A, n, win.wlo, win.Wg, st);
+    const float *counts = kind == 0 ? d_data : nullptr;
+    if (plain) launch_to_window(counts, rows, wt, nslices * A, A, n, win.wlo, win.Wg, st);
+    else launch_to_window4(counts, rows, wt, nslices, A, n, win.wlo, win.Wg, st);
     bl.img = den;
     bl.den = nullptr;
     launch_backproject(bl, st);
@@ -718,17 +738,11 @@ void em_chunk(DeviceState &ds, const EmPrepared &ep, int kind, const float *d_da
     pl.flat = d_flat;
     pl.data = d_data;
     pl.wt = wt;
-    // the projector writes the window rows interleaved by slice, as the
-    // four-slice backprojector stages them: no separate interleave pass per
-    // iteration (margins and slices past the batch stay zero from this clear)
-    pl.windowed = 2;
-    pl.out = static_cast<float *>(bl.il_ws);
-    RAFT_CUDA(cudaMemsetAsync(bl.il_ws, 0, bp_il_bytes(nslices, A, win.Wg, 4), st));
+    pl.windowed = plain ? 1 : 2;
     pl.wlo = win.wlo;
     pl.Wg = win.Wg;
     bl.img = d_obj;
     bl.den = den;
-    bl.il_ready = 1;
     if (d_metrics)
         RAFT_CUDA(cudaMemsetAsync(d_metrics, 0, sizeof(double) * 3 * nslices * (size_t)c.niter, st));
 

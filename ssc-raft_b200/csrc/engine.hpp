@@ -64,9 +64,10 @@ struct FbpPrepared {
     WindowLayout win;
     BpGeo geo;
     const FilterPlan *plan = nullptr;
+    int turns = 1 << 30;   // changes of the backprojector's run axis along the angles
 };
 
-FbpPrepared prepare_fbp(const FbpConfig &cfg, int device);
+FbpPrepared prepare_fbp(const FbpConfig &cfg, int device, const float *h_angles);
 
 // Device-resident FBP of `nslices` slices (filter + backprojection), using
 // the device workspace for the window rows; tables must be set up by

@@ -518,6 +518,39 @@ void launch_project(const ProjLaunch &pl, cudaStream_t st)
     }
 }
 
+// Plain sinogram -> weighted window rows interleaved by slice in groups of four
+// (the bins and slices it does not write stay as they are: zero).
+// sino == nullptr writes the weight itself (back-projection of ones).
+__global__ void to_window4_kernel(const float *__restrict__ sino, float *__restrict__ rows,
+                                  const float *__restrict__ wt, int nslices, int nangles, int nrays, int wlo, int Wg)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= nrays) return;
+    const long long nrow = (long long)((nslices + 3) / 4) * nangles;
+    for (long long r = blockIdx.y; r < nrow; r += gridDim.y) {
+        const int g = (int)(r / nangles), a = (int)(r - (long long)g * nangles);
+        const float w = wt[a];
+        float v[4];
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+            const int k = 4 * g + q;
+            v[q] = k < nslices ? (sino ? sino[((size_t)k * nangles + a) * nrays + i] : 1.f) * w : 0.f;
+        }
+        reinterpret_cast<float4 *>(rows)[r * Wg + (i - wlo)] = make_float4(v[0], v[1], v[2], v[3]);
+    }
+}
+
+void launch_to_window4(const float *sino, float *rows, const float *wt, int nslices, int nangles, int nrays, int wlo,
+                       int Wg, cudaStream_t st)
+{
+    if (nslices <= 0 || nangles <= 0) return;
+    const long long nrow = (long long)((nslices + 3) / 4) * nangles;
+    dim3 grid((nrays + 255) / 256, (unsigned)(nrow < 65535 ? nrow : 65535));
+    count_launch();
+    to_window4_kernel<<<grid, 256, 0, st>>>(sino, rows, wt, nslices, nangles, nrays, wlo, Wg);
+    RAFT_CUDA(cudaGetLastError());
+}
+
 // Plain sinogram -> weighted window rows (the rest of each row stays zero).
 // sino == nullptr writes the weight itself (back-projection of ones).
 __global__ void to_window_kernel(const float *__restrict__ sino, float *__restrict__ rows,

@@ -2,7 +2,8 @@
 // and shared-memory mbarriers used by the backprojector's staging pipeline.
 //
 // Only plain (non-multicast) bulk copies from this GPU's global memory are
-// issued; every wait on an mbarrier is bounded.
+// issued; every wait on an mbarrier is bounded.  Also the two-lane FP32
+// instructions of the backprojector and the projector.
 #pragma once
 #include <cstdint>
 
@@ -64,6 +65,37 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t *bar, uint32_t parity
     for (uint32_t it = 0; it < limit; ++it)
         if (mbar_try_wait(bar, parity)) return true;
     return false;
+}
+
+using u64 = unsigned long long;
+__device__ __forceinline__ u64 pack2(float a, float b)
+{
+    u64 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ void unpack2(u64 v, float &a, float &b)
+{
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
+}
+// two-lane FP32 instructions; each lane rounds (and flushes) as the scalar one
+__device__ __forceinline__ u64 add2(u64 a, u64 b)
+{
+    u64 r;
+    asm("add.rn.ftz.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ u64 mul2(u64 a, u64 b)
+{
+    u64 r;
+    asm("mul.rn.ftz.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ u64 fma2(u64 a, u64 b, u64 c)
+{
+    u64 r;
+    asm("fma.rn.ftz.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
 }
 
 }  // namespace raft

@@ -121,6 +121,7 @@ struct WindowLayout {
     int Wg = 0;       // stored elements per row (multiple of the 16-byte granule)
     int W = 0;        // staged elements per angle per tile
     int align = 4;    // element alignment of a staged window start
+    int Wrun = 0;     // staged elements of the run kernel's 32 x 32 tiles
 };
 
 // Launch-time tile configuration of the backprojector.
@@ -160,16 +161,23 @@ struct BpLaunch {
     const float *cs = nullptr, *sn = nullptr;     // FP32 angle tables
     const double *csd = nullptr, *snd = nullptr;  // FP64 angle tables
     int *err = nullptr;                           // device error flag
-    // optional workspace of bp_il_bytes(): lets launches of four slices per
-    // CTA read the rows interleaved by slice (made here from filt)
-    void *il_ws = nullptr;
-    // 1: il_ws already holds the rows interleaved by slice (filt unused);
-    //    only four-slice shapes run
+    // 1: il_ws holds the rows interleaved by slice in groups of four
+    //    (bp_il_bytes; filt unused)
     int il_ready = 0;
+    const void *il_ws = nullptr;
+    // changes of the run axis along the angle list (bp_run_turns)
+    int turns = 1 << 30;
 };
 
 void launch_backproject(const BpLaunch &bl, cudaStream_t st);
 size_t bp_il_bytes(int nslices, int nangles, int Wg, int esize);
+// Times the run axis changes between neighbouring angles, and whether
+// interleaved rows go through the run kernel (which takes linear
+// interpolation's FP32 rows as single floats).
+int bp_run_turns(const float *angles, int nangles);
+bool bp_runs_ok(const BpGeo &g, int geometry, int nangles, int turns);
+// Whether a launch of nslices slices takes plain rows to the run kernel.
+bool bp_run_plain(const BpGeo &g, int geometry, int store, int nslices, int nangles, int turns);
 // True when RAFT_BP_TUNE forces a shape of fewer than four slices per CTA
 // (which reads plain, not interleaved, rows).
 bool bp_forced_planar();
@@ -244,6 +252,10 @@ void stage_proj_images(ProjLaunch &pl, void *scratch, cudaStream_t st);
 // from flat [nslices][numflats][nrays] and dark [nslices][nrays]; out may equal in.
 void launch_background(const float *in, float *out, const float *flat, const float *dark, int nrays, int nangles,
                        int nslices, int numflats, int is_log, cudaStream_t st);
+
+// As launch_to_window, into rows interleaved by slice in groups of four.
+void launch_to_window4(const float *sino, float *rows, const float *wt, int nslices, int nangles, int nrays, int wlo,
+                       int Wg, cudaStream_t st);
 
 // Copy a plain sinogram into weighted window rows (EM: BP of the counts).
 void launch_to_window(const float *sino, float *rows, const float *wt, int nrows, int nangles,

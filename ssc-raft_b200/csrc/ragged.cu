@@ -115,7 +115,7 @@ extern "C" int raft_ragged_device(int gpu, const raft_request *reqs, int nreq, i
                 c.store = store;
                 FbpReq r;
                 r.idx = i;
-                r.fp = prepare_fbp(c, gpu);
+                r.fp = prepare_fbp(c, gpu, nullptr);
                 r.tab = off;
                 off = a256(off + sizeof(double) * 2 * A + sizeof(float) * 4 * A);
                 r.rows = off;
