@@ -22,6 +22,7 @@
 // reference build produces) so that no template instance can contract them
 // differently.
 #include "raft.hpp"
+#include "ptx.hpp"
 #include "profile.hpp"
 
 #include <cstdlib>
@@ -106,25 +107,57 @@ __device__ __forceinline__ void project_block(const ProjLaunch &p, const int bx,
         auto sample_loop = [&](const float t, const float d0, const float ay0, const float ddx,
                                const float ddy, const int nsamp, const int limx, const int limy) {
             int m = ph;
-            for (; m + 3 * PH < nsamp; m += 4 * PH) {
-                float v[4][S];
+            if constexpr (IL) {
+                // two samples' positions and two slices' sums per instruction (the
+                // lanes round as the scalar instructions do); the sample number is
+                // counted in float, exactly.  39 -> 30 instructions per sample.
+                const u64 d2 = pack2(d0, d0), na2 = pack2(-ay0, -ay0), t2 = pack2(t, t), c2 = pack2(ctheta, ctheta);
+                const u64 s2 = pack2(stheta, stheta), ns2 = pack2(-stheta, -stheta), one2 = pack2(1.f, 1.f);
+                const float rx = __fdividef(1.0f, ddx), ry = __fdividef(1.0f, ddy);   // a / ddx is a times this
+                const u64 rx2 = pack2(rx, rx), ry2 = pack2(ry, ry), step2 = pack2(4.f * PH, 4.f * PH);
+                u64 m01 = pack2((float)ph, (float)(ph + PH)), m23 = pack2((float)(ph + 2 * PH), (float)(ph + 3 * PH));
+                u64 sum[4];
 #pragma unroll
-                for (int u = 0; u < 4; u++) {
-                    const float s = __fmaf_rn((float)(m + u * PH), d0, -ay0);
-                    const float x = __fmaf_rn(t, ctheta, -__fmul_rn(s, stheta));
-                    const float y = __fmaf_rn(t, stheta, __fmul_rn(s, ctheta));
-                    const int X = (int)((x + 1) / ddx);
-                    const int Y = (int)((y + 1) / ddy);
-                    if constexpr (IL) {
-                        // one 32-byte load: the pixel's eight slice values, or
-                        // eight zeros (p.il_zero) for a sample outside the image
-                        const bool in = ((unsigned)X < (unsigned)limx) & ((unsigned)Y < (unsigned)limy);
-                        const unsigned pix = (unsigned)Y * (unsigned)sy + (unsigned)X * (unsigned)sx;
-                        float w[8];
-                        ldg_v8(in ? img + (size_t)pix * 8 : p.il_zero, w);
+                for (int q = 0; q < 4; q++) sum[q] = 0ull;
+                for (; m + 3 * PH < nsamp; m += 4 * PH) {
+                    float w[4][8];
 #pragma unroll
-                        for (int q = 0; q < 8; q++) v[u][q] = w[q];
-                    } else {
+                    for (int h = 0; h < 2; h++) {
+                        const u64 s = fma2(h ? m23 : m01, d2, na2);
+                        const u64 x = mul2(add2(fma2(t2, c2, mul2(s, ns2)), one2), rx2);
+                        const u64 y = mul2(add2(fma2(t2, s2, mul2(s, c2)), one2), ry2);
+                        float xf[2], yf[2];
+                        unpack2(x, xf[0], xf[1]);
+                        unpack2(y, yf[0], yf[1]);
+#pragma unroll
+                        for (int u = 0; u < 2; u++) {
+                            // one 32-byte load: the pixel's eight slice values, or
+                            // eight zeros (p.il_zero) for a sample outside the image
+                            const int X = (int)xf[u], Y = (int)yf[u];
+                            const bool in = ((unsigned)X < (unsigned)limx) & ((unsigned)Y < (unsigned)limy);
+                            const unsigned pix = (unsigned)Y * (unsigned)sy + (unsigned)X * (unsigned)sx;
+                            ldg_v8(in ? img + (size_t)pix * 8 : p.il_zero, w[2 * h + u]);
+                        }
+                    }
+                    m01 = add2(m01, step2);
+                    m23 = add2(m23, step2);
+#pragma unroll
+                    for (int u = 0; u < 4; u++)
+#pragma unroll
+                        for (int q = 0; q < 4; q++) sum[q] = add2(sum[q], pack2(w[u][2 * q], w[u][2 * q + 1]));
+                }
+#pragma unroll
+                for (int q = 0; q < 4; q++) unpack2(sum[q], linesum[2 * q], linesum[2 * q + 1]);
+            } else {
+                for (; m + 3 * PH < nsamp; m += 4 * PH) {
+                    float v[4][S];
+#pragma unroll
+                    for (int u = 0; u < 4; u++) {
+                        const float s = __fmaf_rn((float)(m + u * PH), d0, -ay0);
+                        const float x = __fmaf_rn(t, ctheta, -__fmul_rn(s, stheta));
+                        const float y = __fmaf_rn(t, stheta, __fmul_rn(s, ctheta));
+                        const int X = (int)((x + 1) / ddx);
+                        const int Y = (int)((y + 1) / ddy);
                         // 32-bit pixel index (the launch checks nx * ny < 2^32), predicated loads
                         const bool in = ((unsigned)X < (unsigned)limx) & ((unsigned)Y < (unsigned)limy);
                         const unsigned pix = (unsigned)Y * (unsigned)sy + (unsigned)X * (unsigned)sx;
@@ -135,11 +168,11 @@ __device__ __forceinline__ void project_block(const ProjLaunch &p, const int bx,
                             v[u][q] = val;
                         }
                     }
+#pragma unroll
+                    for (int u = 0; u < 4; u++)
+#pragma unroll
+                        for (int q = 0; q < S; q++) linesum[q] += v[u][q];
                 }
-#pragma unroll
-                for (int u = 0; u < 4; u++)
-#pragma unroll
-                    for (int q = 0; q < S; q++) linesum[q] += v[u][q];
             }
             for (; m < nsamp; m += PH) {
                 const float s = __fmaf_rn((float)m, d0, -ay0);
@@ -398,20 +431,22 @@ void launch_transpose(const float *in, float *out, int nx, int ny, int nslices, 
 // Slice-interleaved copies of groups of 8 planes, row-major and transposed:
 // il[g][y][x][s] = ilT[g][x][y][s] = in[8g + s][y][x] (zero where 8g + s is
 // past the last plane), plus the eight zeros that samples outside the image
-// read.  One 32 x 32 pixel tile of all 8 planes per block.
+// read.  One 32 x TY pixel tile of all 8 planes per block: TY = 32, or 8 where
+// that would leave SMs without a block (301^2: 100 blocks, 10.9 us).
+template <int TY>
 __global__ void __launch_bounds__(256)
 interleave_kernel(const float *__restrict__ in, float *__restrict__ il, float *__restrict__ ilT,
                   float *__restrict__ zero8, int nx, int ny, int nslices)
 {
-    __shared__ float tile[8][32][33];
+    __shared__ float tile[8][TY][33];
     const size_t plane = (size_t)nx * ny;
     const int g = blockIdx.z, tx = threadIdx.x;
     if ((blockIdx.x | blockIdx.y | blockIdx.z | threadIdx.y) == 0 && tx < 8) zero8[tx] = 0.f;
-    const int bx = blockIdx.x * 32, by = blockIdx.y * 32;
+    const int bx = blockIdx.x * 32, by = blockIdx.y * TY;
 #pragma unroll
     for (int s = 0; s < 8; s++) {
         const int k = g * 8 + s;
-        for (int r = threadIdx.y; r < 32; r += blockDim.y) {
+        for (int r = threadIdx.y; r < TY; r += 8) {
             const int y = by + r, x = bx + tx;
             tile[s][r][tx] = (k < nslices && x < nx && y < ny) ? in[(size_t)k * plane + (size_t)y * nx + x] : 0.f;
         }
@@ -419,37 +454,43 @@ interleave_kernel(const float *__restrict__ in, float *__restrict__ il, float *_
     __syncthreads();
     float *o = il + (size_t)g * plane * 8;
     float *oT = ilT + (size_t)g * plane * 8;
-    for (int r = threadIdx.y; r < 32; r += blockDim.y) {
-        int y = by + r, x = bx + tx;
-        if (x < nx && y < ny) {
-            float4 *d = reinterpret_cast<float4 *>(o + ((size_t)y * nx + x) * 8);
-            d[0] = make_float4(tile[0][r][tx], tile[1][r][tx], tile[2][r][tx], tile[3][r][tx]);
-            d[1] = make_float4(tile[4][r][tx], tile[5][r][tx], tile[6][r][tx], tile[7][r][tx]);
-        }
-        x = bx + r;
-        y = by + tx;
-        if (x < nx && y < ny) {
-            float4 *d = reinterpret_cast<float4 *>(oT + ((size_t)x * ny + y) * 8);
-            d[0] = make_float4(tile[0][tx][r], tile[1][tx][r], tile[2][tx][r], tile[3][tx][r]);
-            d[1] = make_float4(tile[4][tx][r], tile[5][tx][r], tile[6][tx][r], tile[7][tx][r]);
-        }
+    auto put = [&](float *p, int r, int c) {
+        float4 *d = reinterpret_cast<float4 *>(p);
+        d[0] = make_float4(tile[0][r][c], tile[1][r][c], tile[2][r][c], tile[3][r][c]);
+        d[1] = make_float4(tile[4][r][c], tile[5][r][c], tile[6][r][c], tile[7][r][c]);
+    };
+    for (int r = threadIdx.y; r < TY; r += 8) {
+        const int y = by + r, x = bx + tx;
+        if (x < nx && y < ny) put(o + ((size_t)y * nx + x) * 8, r, tx);
+    }
+    // transposed: TY consecutive y per x
+    for (int e = threadIdx.y * 32 + tx; e < 32 * TY; e += 256) {
+        const int c = e / TY, r = e % TY, x = bx + c, y = by + r;
+        if (x < nx && y < ny) put(oT + ((size_t)x * ny + y) * 8, r, c);
     }
 }
 
-static bool use_interleaved(int nslices) { return nslices >= 8; }
+// Interleaved copies from three slices on: a group of eight costs the same with
+// fewer, 36 us against 71 us planar for 3 x 301^2 x 257 (two planar slices cost
+// about as much as a group).  Their 16 planes are not taken for few planes of
+// a size where they would claim a good part of the memory.
+static bool use_interleaved(int nx, int ny, int nslices)
+{
+    return nslices >= 8 || (nslices >= 3 && (size_t)nx * ny <= ((size_t)1 << 26));
+}
 
 size_t proj_scratch_bytes(int nx, int ny, int nslices)
 {
     const size_t plane = (size_t)nx * ny * sizeof(float);
     if (nslices <= 0) return 16;
-    if (use_interleaved(nslices)) return 2 * (size_t)((nslices + 7) / 8) * 8 * plane + 8 * sizeof(float);
+    if (use_interleaved(nx, ny, nslices)) return 2 * (size_t)((nslices + 7) / 8) * 8 * plane + 8 * sizeof(float);
     return (size_t)nslices * plane;
 }
 
 void stage_proj_images(ProjLaunch &pl, void *scratch, cudaStream_t st)
 {
     if (pl.nslices <= 0) return;
-    if (use_interleaved(pl.nslices)) {
+    if (use_interleaved(pl.nx, pl.ny, pl.nslices)) {
         // the projector indexes a pixel of the interleaved copies in 32 bits
         RAFT_CHECK((size_t)pl.nx * pl.ny <= 0xffffffffull, "projector: image plane above 2^32 pixels");
         const int G = (pl.nslices + 7) / 8;
@@ -457,8 +498,13 @@ void stage_proj_images(ProjLaunch &pl, void *scratch, cudaStream_t st)
         float *ilT = il + (size_t)G * 8 * pl.nx * pl.ny;
         float *zero8 = ilT + (size_t)G * 8 * pl.nx * pl.ny;
         count_launch();
-        dim3 grid((pl.nx + 31) / 32, (pl.ny + 31) / 32, G);
-        interleave_kernel<<<grid, dim3(32, 8), 0, st>>>(pl.img, il, ilT, zero8, pl.nx, pl.ny, pl.nslices);
+        const unsigned bx = (pl.nx + 31) / 32, by = (pl.ny + 31) / 32;
+        if ((long long)bx * by * G < 2 * 148)
+            interleave_kernel<8><<<dim3(bx, (pl.ny + 7) / 8, G), dim3(32, 8), 0, st>>>(pl.img, il, ilT, zero8, pl.nx, pl.ny,
+                                                                                    pl.nslices);
+        else
+            interleave_kernel<32><<<dim3(bx, by, G), dim3(32, 8), 0, st>>>(pl.img, il, ilT, zero8, pl.nx, pl.ny,
+                                                                        pl.nslices);
         RAFT_CUDA(cudaGetLastError());
         pl.il = il;
         pl.ilT = ilT;

@@ -244,7 +244,7 @@ void launch_transpose(const float *in, float *out, int nx, int ny, int nslices, 
 // Scratch bytes the projector's re-laid-out images need for nslices planes.
 size_t proj_scratch_bytes(int nx, int ny, int nslices);
 // Write the re-laid-out copies of pl.img into `scratch` (proj_scratch_bytes):
-// slice-interleaved groups of 8 (pl.il / pl.ilT) when there are 8 or more
+// slice-interleaved groups of 8 (pl.il / pl.ilT) when there are 3 or more
 // planes, else a transposed copy (pl.imgT).  Issued on st.
 void stage_proj_images(ProjLaunch &pl, void *scratch, cudaStream_t st);
 
