@@ -186,6 +186,9 @@ static void run_pipeline(DeviceState &ds, int nslices, int chunk, size_t in_ps, 
     // page-locked caller buffers are transferred directly; pageable ones are
     // staged through the device's pinned buffers by host threads
     const bool pin_src = is_pinned(host_in), pin_dst = is_pinned(host_out);
+    // staging copies are host work that the device can hide: at least three
+    // chunks (of whole four-slice groups) where there are slices for them
+    if (!pin_src || !pin_dst) chunk = std::min(chunk, std::max(4, (nslices / 3 + 3) / 4 * 4));
     void *din[2], *dout[2], *pin[2] = {nullptr, nullptr}, *pout[2] = {nullptr, nullptr};
     for (int b = 0; b < 2; b++) {
         din[b] = ds.sino[b].get(in_ps * chunk);
