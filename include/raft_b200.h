@@ -291,6 +291,10 @@ int raft_unet_conv_wgrad(const void *dy, const void *x0, int C0, const void *x1,
                          float *dbias, int N, int H, int W, int Cout, void *stream);
 int raft_unet_flip_weights(const void *w, void *wt, int Cout, int Cin, void *stream);
 int raft_unet_relu_bwd(const void *y, const void *dy, void *dpre, size_t n, void *stream);
+/* raft_unet_relu_bwd on [pixels][C] with the bias gradient: dbias[c] += sum over pixels of
+ * dpre, in a fixed order.  C a power of two from 8 to 256, 16-byte aligned tensors. */
+int raft_unet_relu_bwd_bias(const void *y, const void *dy, void *dpre, float *dbias, size_t pixels, int C,
+                            void *stream);
 int raft_unet_pool(int backward, const void *src, void *dst, int N, int H, int W, int C, void *stream);
 int raft_unet_upsample(int backward, const void *src, void *dst, int N, int H, int W, int C, void *stream);
 int raft_unet_input(const float *img, const float *scale, void *x, int N, int H, int W, int C, void *stream);

@@ -358,6 +358,8 @@ int conv3x3_tc_error();
 int conv3x3_wgrad_tc(const void *dy, const void *x0, int C0, const void *x1, int C1, float *dw, float *dbias, int N,
                      int H, int W, int Cout, cudaStream_t st);
 void conv3x3_wgrad_tc_set_nine(int on);
+// ReLU backward with the bias gradient (unet_tc.cu); 0 = launched, 1 = error.
+int relu_bwd_bias(const void *y, const void *dy, void *dpre, float *dbias, long long P, int C, cudaStream_t st);
 void conv3x3_tc_set_halo(int on);
 
 }  // namespace raft

@@ -120,14 +120,14 @@ __device__ __forceinline__ uint64_t umma_desc(uint32_t saddr, uint32_t sbo_bytes
            ((uint64_t)1 << 46) | ((uint64_t)layout << 61);
 }
 
-// Halo tiles (the level-0 layers: 32 channels in, 32 out, W >= 128): one tile =
-// 4 rows x 128 pixels (MT = 4 MMA blocks); a k-block is one 32-channel chunk
-// with all nine taps.  The input arrives once per k-block as one (4+2) x 136
+// Halo tiles (layers with few channels, W >= 128): one tile = MT rows x 128
+// pixels (MT MMA blocks); a k-block is one 32-channel chunk
+// with all nine taps.  The input arrives once per k-block as one (MT+2) x 136
 // pixel halo box (64-byte swizzled rows), so a tap's 128-row operand starts
 // at row (mt + ky + 1) * 136 + kx + 1 of it: a descriptor offset, no reload.
 // The MMA applies the swizzle to absolute shared-memory addresses, as the TMA
 // unit does (base offset 0 at any row; checked against the oracle).
-constexpr int HB_W = 136, HB_H = 6, HB_ROWS = HB_W * HB_H;
+constexpr int HB_W = 136;             // box width; MT + 2 rows high
 
 // ------------------------------------------------------------------- TMA
 __device__ __forceinline__ void tma_load_4d(void *dst, const CUtensorMap *map, int c0, int c1, int c2, int c3,
@@ -190,17 +190,18 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
     conv3x3_tc_kernel(const __grid_constant__ CUtensorMap mx0, const __grid_constant__ CUtensorMap mx1,
                       const __grid_constant__ CUtensorMap mw, const TcArgs a)
 {
-    static_assert(!HALO || (BN == 32 && KC == 32 && MT == 4), "halo tiles: 32 -> 32 channels, 4 MMA blocks");
+    static_assert(!HALO || KC == 32, "halo tiles: 32-channel chunks");
     constexpr int A_PART = TC_M * KC * 2;                  // one 128-row MMA operand
     constexpr int B_TAP = BN * KC * 2;                     // one tap's weights
-    constexpr int A_BYTES = HALO ? HB_ROWS * KC * 2 : MT * A_PART;
+    constexpr int A_BYTES = HALO ? HB_W * (MT + 2) * KC * 2 : MT * A_PART;
     // halo tiles keep every tap's weights resident (loaded once per CTA); the
     // stages carry the input boxes only
     constexpr int B_BYTES = HALO ? 0 : B_TAP, STAGE = A_BYTES + B_BYTES;
     constexpr uint32_t SBO = 8 * KC * 2;                   // one 8-row swizzle atom
     constexpr uint32_t LAYOUT = KC == 64 ? 2u : 4u;        // 128-byte / 64-byte swizzle
     constexpr uint32_t ACC = MT * BN;                      // TMEM columns of one accumulator buffer
-    constexpr uint32_t TMEM_COLS = 2 * ACC < 32 ? 32 : 2 * ACC;
+    // columns are allocated in powers of two
+    constexpr uint32_t TMEM_COLS = 2 * ACC <= 64 ? 64 : 2 * ACC <= 128 ? 128 : 2 * ACC <= 256 ? 256 : 512;
     static_assert(2 * ACC <= 512, "two accumulator buffers must fit in TMEM");
     // lanes of the MMA warp that issue: halo tiles issue their MT blocks from MT
     // lanes at once (one warp instruction, MT MMAs); each issuing lane commits
@@ -496,14 +497,15 @@ bool encode_act(CUtensorMap *m, const void *ptr, int C, int N, int H, int W, int
                CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-// halo-tile instance: 32 -> 32 channels, two stages of one halo box and nine weight boxes
+// halo-tile instance: BN output channels, three stages of one halo box, resident weights
+template <int BN, int MT>
 int launch_tc_halo(const CUtensorMap &m0, const CUtensorMap &m1, const CUtensorMap &mw, const TcArgs &a,
                    cudaStream_t st)
 {
-    constexpr int STAGE = HB_ROWS * 32 * 2, ST = 3;
+    constexpr int STAGE = HB_W * (MT + 2) * 32 * 2, ST = 3;
     static_assert(STAGE % 1024 == 0, "stage alignment");
-    const size_t SMEM = (size_t)ST * STAGE + (size_t)9 * ((a.C0 + a.C1) / 32) * 32 * 32 * 2 + 1024 + 256;
-    auto kern = conv3x3_tc_kernel<32, 32, 4, ST, true>;
+    const size_t SMEM = (size_t)ST * STAGE + (size_t)9 * ((a.C0 + a.C1) / 32) * BN * 32 * 2 + 1024 + 256;
+    auto kern = conv3x3_tc_kernel<BN, 32, MT, ST, true>;
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM) != cudaSuccess) return 1;
     cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
     int dev = 0, sms = 148, occ = 1;
@@ -1005,17 +1007,34 @@ int launch_wgrad_tc9(const CUtensorMap &m0, const CUtensorMap &m1, const CUtenso
     return cudaGetLastError() == cudaSuccess ? 0 : 1;
 }
 
-// dw[co][r] += sum over splits of part[split][r][co], r = tap * Cin + ci < rows
-__global__ void wgrad_reduce_kernel(const float *__restrict__ part, float *__restrict__ dw, int splits, int rows,
-                                    int prow, int Cout)
+// dw[co][r] += sum over splits of part[split][r][co], r = tap * Cin + ci < rows.
+// A block takes four r and 32 co; its eight warps share the splits (warp w sums
+// w, w + 8, ...), whose sums are added in warp order.  With one thread walking all
+// splits of an element, 32 -> 32 channels (9216 elements, 148 splits) had 36
+// blocks of dependent loads: 17 us.
+__global__ void __launch_bounds__(256) wgrad_reduce_kernel(const float *__restrict__ part, float *__restrict__ dw,
+                                                           int splits, int rows, int prow, int Cout)
 {
-    const size_t n = (size_t)rows * Cout;
-    for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < n; e += (size_t)gridDim.x * blockDim.x) {
-        const int co = (int)(e % Cout);
-        const int r = (int)(e / Cout);
-        float acc = 0.f;
-        for (int sp = 0; sp < splits; ++sp) acc += part[((size_t)sp * prow + r) * Cout + co];
-        dw[(size_t)co * rows + r] += acc;
+    __shared__ float red[8][4][32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int r0 = blockIdx.x * 4, c0 = blockIdx.y * 32;
+    const size_t stride = (size_t)prow * Cout;
+    const float *src = part + (size_t)r0 * Cout + c0 + lane;
+    float acc[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll 4
+    for (int sp = warp; sp < splits; sp += 8)
+#pragma unroll
+        for (int q = 0; q < 4; q++)
+            if (r0 + q < rows) acc[q] += __ldcs(src + sp * stride + (size_t)q * Cout);
+#pragma unroll
+    for (int q = 0; q < 4; q++) red[warp][q][lane] = acc[q];
+    __syncthreads();
+    if (threadIdx.x < 128) {
+        const int q = threadIdx.x & 3, co = threadIdx.x >> 2;
+        float sum = 0.f;
+#pragma unroll
+        for (int w = 0; w < 8; w++) sum += red[w][q][co];
+        if (r0 + q < rows) dw[(size_t)(c0 + co) * rows + r0 + q] += sum;
     }
 }
 
@@ -1040,6 +1059,46 @@ bias_partial_kernel(const bf16 *__restrict__ dy, float *__restrict__ part, long 
                 acc[2 * q] += f.x;
                 acc[2 * q + 1] += f.y;
             }
+        }
+    }
+#pragma unroll
+    for (int q = 0; q < 8; q++) red[threadIdx.x * 8 + q] = acc[q];
+    __syncthreads();
+    if (threadIdx.x < Cout) {
+        const int co = threadIdx.x, c = co / 8, q = co % 8;
+        float sum = 0.f;
+        for (int l = 0; l < L; ++l) sum += red[(l * g8 + c) * 8 + q];
+        part[(size_t)blockIdx.x * Cout + co] = sum;
+    }
+}
+
+// ReLU backward, dpre = dy where y > 0, with the bias gradient's per-block sums of
+// dpre in the same pass (bias_partial_kernel's ranges and order, so the same bits):
+// a pass of its own over dpre took 25 us per 134 MB layer.
+__global__ void __launch_bounds__(256)
+relu_bwd_bias_kernel(const bf16 *__restrict__ y, const bf16 *__restrict__ dy, bf16 *__restrict__ dpre,
+                     float *__restrict__ part, long long P, int Cout, long long per)
+{
+    __shared__ float red[256 * 8];
+    const int g8 = Cout / 8, L = 256 / g8, c8 = threadIdx.x % g8, pl = threadIdx.x / g8;
+    const long long p0 = (long long)blockIdx.x * per, p1 = p0 + per < P ? p0 + per : P;
+    float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+    if (pl < L) {
+#pragma unroll 4
+        for (long long p = p0 + pl; p < p1; p += L) {
+            const size_t o = (size_t)p * Cout + 8 * c8;
+            const uint4 a = __ldcs(reinterpret_cast<const uint4 *>(y + o));
+            const uint4 g = __ldcs(reinterpret_cast<const uint4 *>(dy + o));
+            const uint32_t av[4] = {a.x, a.y, a.z, a.w}, gv[4] = {g.x, g.y, g.z, g.w};
+            uint32_t r[4];
+#pragma unroll
+            for (int q = 0; q < 4; q++) {
+                const int16_t lo = (int16_t)(av[q] & 0xffffu), hi = (int16_t)(av[q] >> 16);
+                r[q] = (lo > 0 ? (gv[q] & 0xffffu) : 0u) | (hi > 0 ? (gv[q] & 0xffff0000u) : 0u);
+                acc[2 * q] += __uint_as_float(r[q] << 16);
+                acc[2 * q + 1] += __uint_as_float(r[q] & 0xffff0000u);
+            }
+            *reinterpret_cast<uint4 *>(dpre + o) = make_uint4(r[0], r[1], r[2], r[3]);
         }
     }
 #pragma unroll
@@ -1180,21 +1239,26 @@ int conv3x3_tc(const void *x0, int C0, const void *x1, int C1, const void *w, co
     cudaGetDevice(&dev);
     a.err = tc_err_flag(dev);
     CUtensorMap m0, m1, mw;
-    if (g_halo && Cout == 32 && KC == 32 && W >= TC_M && C0 + C1 <= 96) {
-        // halo tiles: 4 rows x 128 pixels, the taps served from one box per channel chunk
+    // Halo tiles: 4 rows x 128 pixels, the taps served from one box per 32-channel
+    // chunk, all output channels in one MMA: 32 channels from up to 96, and 64 or 96
+    // (two rows: four would not fit TMEM twice) from 32.  8 x 512^2, 32 -> 96: 377 us
+    // as three passes of 32 channels over per-tap boxes.
+    if (g_halo && W >= TC_M && ((Cout == 32 && C0 + C1 <= 96) || ((Cout == 64 || Cout == 96) && C0 + C1 == 32))) {
         TcArgs h = a;
         h.BW = TC_M;
-        h.BH = 4;
+        h.BH = Cout == 96 ? 2 : 4;
         h.n_xb = (W + TC_M - 1) / TC_M;
-        h.n_yb = (H + 3) / 4;
+        h.n_yb = (H + h.BH - 1) / h.BH;
         h.n_co = 1;
         const long long ht = (long long)N * h.n_yb * h.n_xb;
-        if (ht > 0 && ht <= (1LL << 30) && encode_act(&m0, x0, C0, N, H, W, 32, HB_W, HB_H) &&
-            (C1 == 0 || encode_act(&m1, x1, C1, N, H, W, 32, HB_W, HB_H)) &&
-            encode_w(&mw, w, Cout, C0 + C1, 32, 32)) {
+        if (ht > 0 && ht <= (1LL << 30) && encode_act(&m0, x0, C0, N, H, W, 32, HB_W, h.BH + 2) &&
+            (C1 == 0 || encode_act(&m1, x1, C1, N, H, W, 32, HB_W, h.BH + 2)) &&
+            encode_w(&mw, w, Cout, C0 + C1, 32, Cout)) {
             if (C1 == 0) m1 = m0;
             h.tiles = (int)ht;
-            return launch_tc_halo(m0, m1, mw, h, st);
+            if (Cout == 96) return launch_tc_halo<96, 2>(m0, m1, mw, h, st);
+            if (Cout == 64) return launch_tc_halo<64, 4>(m0, m1, mw, h, st);
+            return launch_tc_halo<32, 4>(m0, m1, mw, h, st);
         }
     }
     if (!encode_act(&m0, x0, C0, N, H, W, KC, a.BW, a.BH)) return 2;
@@ -1285,8 +1349,7 @@ int conv3x3_wgrad_tc(const void *dy, const void *x0, int C0, const void *x1, int
     if (rc) return rc;
     const int rows = 9 * Cin;
     count_launch();
-    wgrad_reduce_kernel<<<(unsigned)std::min<size_t>(((size_t)rows * Cout + 255) / 256, 148 * 16), 256, 0, st>>>(
-        a.part, dw, a.splits, rows, prow, Cout);
+    wgrad_reduce_kernel<<<dim3((rows + 3) / 4, Cout / 32), 256, 0, st>>>(a.part, dw, a.splits, rows, prow, Cout);
     if (cudaGetLastError() != cudaSuccess) return 1;
     if (dbias) {
         float *bp = ws + part_floats;
@@ -1298,6 +1361,23 @@ int conv3x3_wgrad_tc(const void *dy, const void *x0, int C0, const void *x1, int
         if (cudaGetLastError() != cudaSuccess) return 1;
     }
     return 0;
+}
+
+int relu_bwd_bias(const void *y, const void *dy, void *dpre, float *dbias, long long P, int C, cudaStream_t st)
+{
+    if (P < 1 || C < 8 || C > 256 || 256 % C || (((uintptr_t)y | (uintptr_t)dy | (uintptr_t)dpre) & 15)) return 1;
+    int dev = 0, sms = 148;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    const int blk = (int)std::min<long long>(4 * sms, std::max(1LL, P / 256));
+    float *part = wgrad_workspace(dev, (size_t)blk * C);
+    if (!part) return 1;
+    count_launch();
+    relu_bwd_bias_kernel<<<blk, 256, 0, st>>>((const bf16 *)y, (const bf16 *)dy, (bf16 *)dpre, part, P, C,
+                                              (P + blk - 1) / blk);
+    count_launch();
+    bias_reduce_kernel<<<C, 256, 0, st>>>(part, dbias, blk, C);
+    return cudaGetLastError() == cudaSuccess ? 0 : 1;
 }
 
 // Reads and clears the tensor-core convolution's error flag of the current device

@@ -27,6 +27,7 @@ libraft.raft_unet_conv_fwd.argtypes = [_P, _I, _P, _I, _P, _P, _P, _P, _I, _I, _
 libraft.raft_unet_conv_wgrad.argtypes = [_P, _P, _I, _P, _I, _P, _P, _I, _I, _I, _I, _P]
 libraft.raft_unet_flip_weights.argtypes = [_P, _P, _I, _I, _P]
 libraft.raft_unet_relu_bwd.argtypes = [_P, _P, _P, _Z, _P]
+libraft.raft_unet_relu_bwd_bias.argtypes = [_P, _P, _P, _P, _Z, _I, _P]
 libraft.raft_unet_pool.argtypes = [_I, _P, _P, _I, _I, _I, _I, _P]
 libraft.raft_unet_upsample.argtypes = [_I, _P, _P, _I, _I, _I, _I, _P]
 libraft.raft_unet_input.argtypes = [_P, _P, _P, _I, _I, _I, _I, _P]
@@ -41,7 +42,7 @@ libraft.raft_unet_set_conv_path.argtypes = [_I]
 libraft.raft_unet_set_conv_halo.argtypes = [_I]
 libraft.raft_unet_set_wgrad_nine.argtypes = [_I]
 libraft.raft_unet_conv_error.argtypes = []
-for _f in ("raft_unet_set_conv_path", "raft_unet_set_conv_halo", "raft_unet_set_wgrad_nine", "raft_unet_conv_error", "raft_unet_conv_fwd", "raft_unet_conv_wgrad", "raft_unet_flip_weights", "raft_unet_relu_bwd",
+for _f in ("raft_unet_set_conv_path", "raft_unet_set_conv_halo", "raft_unet_set_wgrad_nine", "raft_unet_conv_error", "raft_unet_conv_fwd", "raft_unet_conv_wgrad", "raft_unet_flip_weights", "raft_unet_relu_bwd", "raft_unet_relu_bwd_bias",
            "raft_unet_pool", "raft_unet_upsample", "raft_unet_input", "raft_unet_input_conv", "raft_unet_input_wgrad",
            "raft_unet_head",
            "raft_unet_mse",
@@ -164,8 +165,8 @@ class UNet:
         _, c0, c1, co = next(l for l in self.LAYERS if l[0] == name)
         st = self._st()
         dpre = torch.empty_like(gy)
-        _ok(libraft.raft_unet_relu_bwd(_p(y), _p(gy), _p(dpre), gy.numel(), st), "relu_bwd")
-        _ok(libraft.raft_unet_conv_wgrad(_p(dpre), _p(x0), c0, _p(x1), c1, _p(self.gw[name]), _p(self.gb[name]),
+        _ok(libraft.raft_unet_relu_bwd_bias(_p(y), _p(gy), _p(dpre), _p(self.gb[name]), N * H * W, co, st), "relu_bwd")
+        _ok(libraft.raft_unet_conv_wgrad(_p(dpre), _p(x0), c0, _p(x1), c1, _p(self.gw[name]), None,
                                          N, H, W, co, st), "wgrad " + name)
         if not need_dx:
             return None, None
