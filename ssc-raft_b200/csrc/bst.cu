@@ -93,22 +93,38 @@ __global__ void __launch_bounds__(512) bst_rows_kernel(const BstArgs p)
     const bool has1 = a1 < p.A;
     const float *s0 = p.tomo + ((size_t)slice * p.A + a0) * p.N;
     const float *s1 = s0 + p.N;
-    for (int n = threadIdx.x; n < p.Np; n += blockDim.x) {
+    auto padded = [=](int n) {
         const int i = min(max(n - p.off, 0), p.N - 1);
-        z[n] = make_float2(__ldg(s0 + i), has1 ? __ldg(s1 + i) : 0.f);
-    }
-    __syncthreads();
+        return make_float2(__ldg(s0 + i), has1 ? __ldg(s1 + i) : 0.f);
+    };
     float sgn1 = 1.f;   // the second row is sgn1 * z.y
-    if (p.G) {
-        float2 *r = bst_fft<NF>(z, sm_bst + p.M, p.pN);
-        for (int k = threadIdx.x; k < p.Np; k += blockDim.x) {
-            const float2 g = cmul(r[k], __ldg(&p.G[k]));
-            r[k] = make_float2(g.x, -g.y);
-        }
-        __syncthreads();
+    if (NF > 0 && p.G) {
+        // transform, filter weights and conjugation in the last pass; then the
         // forward transform of the conjugate = conjugate of the inverse
-        z = bst_fft<NF>(r, r == sm_bst ? sm_bst + p.M : sm_bst, p.pN);
+        if constexpr (NF > 0) {
+            float2 *A = sm_bst, *B = sm_bst + p.M, *X = cfft_out_buffer<NF>() ? B : A, *O = X == A ? B : A;
+            const float2 *G = p.G;
+            cfft_stream<NF>(A, B, padded, [=](int k, float2 v) {
+                const float2 g = cmul(v, __ldg(&G[k]));
+                X[k] = make_float2(g.x, -g.y);
+            });
+            __syncthreads();
+            z = cfft_smem<NF>(X, O);
+        }
         sgn1 = -1.f;
+    } else {
+        for (int n = threadIdx.x; n < p.Np; n += blockDim.x) z[n] = padded(n);
+        __syncthreads();
+        if (p.G) {
+            float2 *r = bst_fft<NF>(z, sm_bst + p.M, p.pN);
+            for (int k = threadIdx.x; k < p.Np; k += blockDim.x) {
+                const float2 g = cmul(r[k], __ldg(&p.G[k]));
+                r[k] = make_float2(g.x, -g.y);
+            }
+            __syncthreads();
+            z = bst_fft<NF>(r, r == sm_bst ? sm_bst + p.M : sm_bst, p.pN);
+            sgn1 = -1.f;
+        }
     }
     // two buffers of M elements: the filtered pair z, and the other one.  The
     // second row's half-rays are parked in its own (not yet written) polar row
@@ -124,20 +140,30 @@ __global__ void __launch_bounds__(512) bst_rows_kernel(const BstArgs p)
             park[idx] = make_float2(w * sgn1 * z[c - 1 - idx].y, w * sgn1 * z[c + idx].y);
         }
     for (int r = 0; r < (has1 ? 2 : 1); r++) {
-        for (int idx = threadIdx.x; idx < p.L; idx += blockDim.x) {
-            float2 h = make_float2(0.f, 0.f);
-            if (idx < half) {
-                if (r == 0) {
-                    const float w = idx == 0 ? 0.5f * p.w_half : p.w_half;
-                    h = make_float2(w * z[c - 1 - idx].x, w * z[c + idx].x);
-                } else {
-                    h = park[idx];       // written by this same thread above
-                }
+        auto halves = [=](int idx) {   // both half-rays of row r, zero-padded
+            if (idx >= half) return make_float2(0.f, 0.f);
+            if (r) return park[idx];
+            const float w = idx == 0 ? 0.5f * p.w_half : p.w_half;
+            return make_float2(w * z[c - 1 - idx].x, w * z[c + idx].x);
+        };
+        const float2 *H;
+        if constexpr (NF > 0) {
+            // the first pass reads z (row 0) or the parked row and writes fa; the
+            // barrier orders the parked values, written by other threads, and the
+            // last reads of fa
+            __syncthreads();
+            float2 *out = cfft_out_buffer<NF>() ? fa : fb;
+            cfft_passes<NF, 0, 1>(fb, fa, CEachIn<NF, decltype(halves)>{halves}, CPlainLast{out});
+            __syncthreads();
+            H = out;
+        } else {
+            for (int idx = threadIdx.x; idx < p.L; idx += blockDim.x) {
+                // r = 1: written by this same thread above
+                fa[idx] = halves(idx);
             }
-            fa[idx] = h;
+            __syncthreads();
+            H = bst_fft<NF>(fa, fb, p.pL);
         }
-        __syncthreads();
-        const float2 *H = bst_fft<NF>(fa, fb, p.pL);
         float2 *frow = p.polar + pb + (size_t)(a0 + r) * p.Lh;           // left half-ray (theta + pi)
         float2 *rrow = p.polar + pb + (size_t)(p.A + a0 + r) * p.Lh;     // right half-ray (theta)
         for (int k = threadIdx.x; k < p.Lh; k += blockDim.x) {
@@ -232,11 +258,19 @@ __global__ void __launch_bounds__(512) bst_gridrows_kernel(const BstArgs p)
     extern __shared__ float2 sm_bst[];
     const int slice = blockIdx.y, Y = blockIdx.x, S = p.S, H = p.H;
     const float2 *row = p.grid + ((size_t)slice * H + Y) * S;
-    for (int X = threadIdx.x; X < S; X += blockDim.x) sm_bst[X] = __ldcs(row + X);
-    __syncthreads();
-    const float2 *r = bst_fft<NF>(sm_bst, sm_bst + fft_plan_span(p.pS), p.pS);
     float2 *trow = p.T + ((size_t)slice * H + Y) * p.N;
-    for (int i = threadIdx.x; i < p.N; i += blockDim.x) trow[i] = r[p.off + i];
+    if constexpr (NF > 0) {
+        const int off = p.off, N = p.N;
+        cfft_stream<NF>(sm_bst, sm_bst + fft_span(NF), [=](int X) { return __ldcs(row + X); },
+                        [=](int X, float2 v) {
+                            if ((unsigned)(X - off) < (unsigned)N) trow[X - off] = v;
+                        });
+    } else {
+        for (int X = threadIdx.x; X < S; X += blockDim.x) sm_bst[X] = __ldcs(row + X);
+        __syncthreads();
+        const float2 *r = bst_fft<NF>(sm_bst, sm_bst + fft_plan_span(p.pS), p.pS);
+        for (int i = threadIdx.x; i < p.N; i += blockDim.x) trow[i] = r[p.off + i];
+    }
 }
 
 // The image columns are the real parts of the crop columns' forward transforms.
@@ -247,27 +281,54 @@ __global__ void __launch_bounds__(512) bst_cols_kernel(const BstArgs p)
 {
     extern __shared__ float2 sm_bst[];
     const int slice = blockIdx.y, i = (HALF ? 2 : 1) * blockIdx.x, S = p.S, H = p.H;
-    const bool two = HALF && i + 1 < p.N;
-    const float2 *tcol = p.T + (size_t)slice * H * p.N + i;
-    for (int Y = threadIdx.x; Y < H; Y += blockDim.x) {
-        const float2 u = tcol[(size_t)Y * p.N], v = two ? tcol[(size_t)Y * p.N + 1] : make_float2(0.f, 0.f);
-        const int m = Y ? S - Y : 0;
-        if (!HALF) {
-            sm_bst[Y] = u;
-        } else if (m == Y) {   // its own mirror image: real
-            sm_bst[Y] = make_float2(u.x, v.x);
+    const bool two = HALF && i + 1 < p.N, pairs = HALF && p.N % 2 == 0;   // 16-byte aligned pairs of columns
+    const int N = p.N;
+    const float2 *tcol = p.T + (size_t)slice * H * N + i;
+    float *o = p.obj + (size_t)slice * N * N + i;
+    const float scale = p.scale;
+    const int off = p.off;
+    const bool wide = pairs && (reinterpret_cast<uintptr_t>(p.obj) & 7) == 0;   // obj is the caller's
+    auto put = [=](int Y, float2 v) {   // element Y of the transform
+        const int j = Y - off;
+        if ((unsigned)j >= (unsigned)N) return;
+        if (wide) {
+            *reinterpret_cast<float2 *>(o + (size_t)j * N) = make_float2(v.x / scale, v.y / scale);
         } else {
-            sm_bst[Y] = make_float2(u.x - v.y, u.y + v.x);
-            sm_bst[m] = make_float2(u.x + v.y, v.x - u.y);
+            o[(size_t)j * N] = v.x / scale;
+            if (two) o[(size_t)j * N + 1] = v.y / scale;
         }
-    }
-    __syncthreads();
-    const float2 *r = bst_fft<NF>(sm_bst, sm_bst + fft_plan_span(p.pS), p.pS);
-    float *o = p.obj + (size_t)slice * p.N * p.N + i;
-    for (int j = threadIdx.x; j < p.N; j += blockDim.x) {
-        const float2 v = r[p.off + j];
-        o[(size_t)j * p.N] = v.x / p.scale;
-        if (two) o[(size_t)j * p.N + 1] = v.y / p.scale;
+    };
+    if constexpr (NF > 0 && !HALF) {
+        cfft_stream<NF>(sm_bst, sm_bst + fft_span(NF), [=](int Y) { return __ldg(tcol + (size_t)Y * N); }, put);
+    } else {
+#pragma unroll 4
+        for (int Y = threadIdx.x; Y < H; Y += blockDim.x) {
+            float2 u, v = make_float2(0.f, 0.f);
+            if (pairs) {
+                const float4 uv = __ldg(reinterpret_cast<const float4 *>(tcol + (size_t)Y * N));
+                u = make_float2(uv.x, uv.y);
+                v = make_float2(uv.z, uv.w);
+            } else {
+                u = tcol[(size_t)Y * N];
+                if (two) v = tcol[(size_t)Y * N + 1];
+            }
+            const int m = Y ? S - Y : 0;
+            if (!HALF) {
+                sm_bst[Y] = u;
+            } else if (m == Y) {   // its own mirror image: real
+                sm_bst[Y] = make_float2(u.x, v.x);
+            } else {
+                sm_bst[Y] = make_float2(u.x - v.y, u.y + v.x);
+                sm_bst[m] = make_float2(u.x + v.y, v.x - u.y);
+            }
+        }
+        __syncthreads();
+        if constexpr (NF > 0) {
+            cfft_stream<NF>(sm_bst, sm_bst + fft_span(NF), [=](int Y) { return sm_bst[Y]; }, put);
+        } else {
+            const float2 *r = bst_fft<NF>(sm_bst, sm_bst + fft_plan_span(p.pS), p.pS);
+            for (int j = threadIdx.x; j < N; j += blockDim.x) put(off + j, r[off + j]);
+        }
     }
 }
 

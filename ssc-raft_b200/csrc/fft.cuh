@@ -454,6 +454,43 @@ struct CPlainLast {
     template <int R, int NS> __device__ __forceinline__ CPlainOut<R, NS> at() const { return {d}; }
 };
 
+// Last-pass output through f(i, value) for every element i of the result.
+template <int R, int NS, class F>
+struct CEachOut {
+    F f;
+    __device__ __forceinline__ void operator()(int q, int k, const float2 (&v)[R]) const
+    {
+        (void)q;
+#pragma unroll
+        for (int r = 0; r < R; r++) f(k + r * NS, v[r]);
+    }
+};
+template <class F> struct CEachLast {
+    F f;
+    template <int R, int NS> __device__ __forceinline__ CEachOut<R, NS, F> at() const { return {f}; }
+};
+// First-pass input get(i), i the element.
+template <int NP, class G> struct CEachIn {
+    G get;
+    __device__ __forceinline__ float2 operator()(int j, int it, int r) const
+    {
+        (void)it;
+        return get(j + r * (NP / c_factorize(NP).r[0]));
+    }
+};
+
+// NP-point forward transform of get(i), handed to put(i, value): the first pass
+// reads its input and the last one passes on its results from registers, so
+// neither goes through shared memory (the same bits as cfft_smem between a copy
+// in and a copy out).  a and b each hold fft_span(NP) elements; the first pass
+// writes b, the second a, and so on, with a barrier after each but the last: get
+// may read a, and put may write the buffer the last pass does not read.
+template <int NP, class G, class F>
+__device__ __forceinline__ void cfft_stream(float2 *a, float2 *b, const G &get, const F &put)
+{
+    cfft_passes<NP, 0, 1>(a, b, CEachIn<NP, G>{get}, CEachLast<F>{put});
+}
+
 // fft_forward for a compile-time length with blockDim.x == c_fft_threads(NP):
 // the NP values in a (plain order) are transformed, the result (plain order)
 // is left in the returned buffer, a or b, after a barrier.
