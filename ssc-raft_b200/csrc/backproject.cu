@@ -14,9 +14,12 @@
 //     detector grid, the sample at fractional bin u = (t - tmin)/dt is
 //     interpolated between bins floor(u) and floor(u)+1 (zero outside).
 //
-// B200 design.  A CTA owns a 64 x 32 pixel tile of one slice (256 threads,
-// 8 pixels per thread spread so that every warp touches an 8 x 4 pixel
-// block -> one shared-memory wavefront per gather).  Angles stream through a
+// B200 design.  Two kernels with the same per-pixel arithmetic and bits: the run
+// kernel (bp_run.cuh, four neighbouring pixels per thread) where pixels are as wide
+// as detector bins, and the general one described here for everything else.  A CTA
+// owns a 64 x 32 pixel tile of one to four slices (256 threads, 8 pixels per
+// thread spread so that every warp touches an 8 x 4 pixel block -> one
+// shared-memory wavefront per gather).  Angles stream through a
 // two-stage pipeline of 32-angle blocks: for every angle, warp 0 computes the
 // detector window the tile can reach and one lane issues a 1-D bulk copy
 // (cp.async.bulk, the TMA engine) of that window from the filtered rows in

@@ -775,62 +775,82 @@ __global__ void __launch_bounds__(WG_THREADS, 1)
     }
 }
 
-// All nine taps per CTA (Cout <= 128): the CTA owns one 32-channel input chunk
-// and all 288 (tap, channel) rows -- three M = 128 blocks, the third a quarter
-// full -- so a k-block stages the input once as three 66-pixel row boxes
-// (rows y-1..y+1, columns x0-1..x0+64, the TMA zero fill outside the image)
-// and every tap's operand rows are transposed out of them at a column offset.
-// The staging ring is deeper than the operand ring: the loads of several
-// k-blocks are in flight while the tensor cores work through the operands.
-constexpr int WG9_BOX = 66;                   // pixels per row box (64 + the two neighbours)
-constexpr int WG9_BOXB = 4608;                // one box's slot: 66 x 64 bytes, 512-byte aligned
+// All nine taps per CTA (Cout <= 128): the CTA owns one 32-channel input chunk and
+// all 288 (tap, channel) rows, as three accumulators, one per kernel row ky.  The
+// operands stay as the TMA unit lands them: pixel rows of 64 or 128 swizzled bytes
+// are the MMA's MN-major layout (both transpose bits set), so nothing is moved in
+// shared memory.  A ring slot holds one image row segment (64 pixels): the input
+// chunk three times, shifted by kx - 1 pixels (4 KB each, the TMA zero fill outside
+// the image), and dY behind them.  k-blocks run down a column of segments, so a
+// slot serves ky = 0, 1, 2 of three successive k-blocks and each k-block loads one
+// slot; a column's first and last slot carry the halo rows.  An MMA of row ky takes
+// 128 rows = the three shifts of slot y + ky - 1 and, as the unused fourth block of
+// 32, the first 4 KB of that slot's dY: 96 of its 128 accumulator rows are read.
+// Transposing each k-block into K-major operands with ldmatrix / stmatrix had four
+// warps moving 73 KB per k-block.  Bound by the MMA reading 128 x 16 input operands
+// with 64-byte rows, about 120 clocks each (input loaded once with taps as row
+// offsets instead of three times: no change).  Kernel alone before, with the
+// 10 - 15 us reduction after: 8 x 512^2, 32 -> 32: 242 -> 184 us; 96 -> 32: 713 ->
+// 490 us; 8 x 256^2, 192 -> 64: 405 -> 272 us; 8 x 128^2, 384 -> 128: 253 -> 155 us.
+constexpr int WG9_X = WG_KB * 64;             // one shifted copy: 64 pixels x 32 channels
 
 template <int BN>
-__host__ __device__ constexpr int wg9_stg_bytes()
+__host__ __device__ constexpr int wg9_slot_bytes()
 {
-    return (3 * WG9_BOXB + WG_KB * BN * 2 + 1023) / 1024 * 1024;
+    return 3 * WG9_X + WG_KB * BN * 2;
 }
-template <int BN>
-__host__ __device__ constexpr int wg9_op_bytes()
-{
-    return BN * 128 + 288 * 128;             // [opB | opA]; the third block reads 96 rows past opA
-}
-constexpr int WG9_SLACK = 96 * 128;
 
-template <int BN, int STS, int STO>
+// Descriptor of an MN-major operand: lbo bytes between 32- or 64-wide blocks of
+// rows, sbo bytes between groups of eight pixels.
+__device__ __forceinline__ uint64_t umma_desc_mn(uint32_t saddr, uint32_t lbo, uint32_t sbo, uint32_t layout)
+{
+    return (uint64_t)((saddr >> 4) & 0x3FFF) | ((uint64_t)((lbo >> 4) & 0x3FFF) << 16) |
+           ((uint64_t)((sbo >> 4) & 0x3FFF) << 32) | ((uint64_t)1 << 46) | ((uint64_t)layout << 61);
+}
+
+// The epilogue's wait spans all the k-blocks, so its limit grows with them; it ends
+// early when a role that waits for one k-block has given up.
+__device__ __forceinline__ bool wg9_wait_all(uint64_t *bar, long long kblocks, volatile int *abort_flag, int *err)
+{
+    for (long long i = 0; i <= kblocks >> 10; ++i) {
+        for (uint32_t it = 0; it < TC_WAIT_LIMIT; ++it) {
+            if (mbar_try_wait(bar, 0)) return true;
+            if ((it & 255) == 255 && *abort_flag) return false;
+        }
+    }
+    *abort_flag = 1;
+    if (err) atomicExch(err, 1);
+    return false;
+}
+
+template <int BN, int RS>
 __global__ void __launch_bounds__(WG_THREADS, 1)
     wgrad_tc9_kernel(const __grid_constant__ CUtensorMap mx0, const __grid_constant__ CUtensorMap mx1,
                      const __grid_constant__ CUtensorMap mdy, const WgTcArgs a)
 {
-    constexpr int STG = wg9_stg_bytes<BN>(), OPS = wg9_op_bytes<BN>();
-    static_assert(OPS % 1024 == 0 && (BN == 32 || BN == 64 || BN == 128), "layout");
-    constexpr uint32_t IDESC = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) |
-                               ((uint32_t)(TC_M >> 4) << 24);
+    constexpr int SLOT = wg9_slot_bytes<BN>();
+    static_assert(SLOT % 1024 == 0 && (BN == 32 || BN == 64 || BN == 128), "layout");
+    static_assert(RS >= 5, "three slots in use, two to load");
+    constexpr uint32_t IDESC = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 15) | (1u << 16) |
+                               ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(TC_M >> 4) << 24);
     constexpr uint32_t TMEM_COLS = 3 * BN <= 128 ? 128 : 3 * BN <= 256 ? 256 : 512;
-    constexpr uint32_t TX = 3 * WG9_BOX * 64 + WG_KB * BN * 2;
+    // dY: one box of 64-byte rows (BN 32), or BN / 64 boxes of 128-byte rows
+    constexpr uint32_t B_LAYOUT = BN == 32 ? 4 : 2, B_SBO = BN == 32 ? 512 : 1024, B_LBO = WG_KB * 128;
 
     extern __shared__ uint8_t smem_raw[];
-    uint8_t *base = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
-    uint8_t *stg = base;                                   // STS staging slots
-    uint8_t *ops = base + STS * STG;                       // STO operand slots (+ slack)
-    uint64_t *full = reinterpret_cast<uint64_t *>(ops + STO * OPS + WG9_SLACK);
-    uint64_t *sfree = full + STS;
-    uint64_t *opfull = sfree + STS;
-    uint64_t *opfree = opfull + STO;
-    uint64_t *accf = opfree + STO;
+    uint8_t *ring = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+    uint64_t *full = reinterpret_cast<uint64_t *>(ring + RS * SLOT);
+    uint64_t *sfree = full + RS;
+    uint64_t *accf = sfree + RS;
     uint64_t *drain = accf + 1;
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(drain + 1);
     volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (threadIdx.x == 0) {
-        for (int s = 0; s < STS; ++s) {
+        for (int s = 0; s < RS; ++s) {
             mbar_init(&full[s], 1);
-            mbar_init(&sfree[s], 4);
-        }
-        for (int s = 0; s < STO; ++s) {
-            mbar_init(&opfull[s], 4);
-            mbar_init(&opfree[s], 1);
+            mbar_init(&sfree[s], 1);
         }
         mbar_init(accf, 1);
         mbar_init(drain, 1);
@@ -850,9 +870,9 @@ __global__ void __launch_bounds__(WG_THREADS, 1)
     const int cc = (int)(blockIdx.x % (unsigned)cchunks), split = (int)(blockIdx.x / (unsigned)cchunks);
     const long long kb0 = (long long)split * a.kper;
     const long long kb1 = kb0 + a.kper < a.kblocks ? kb0 + a.kper : a.kblocks;
-    const int nk = kb1 > kb0 ? (int)(kb1 - kb0) : 0;
     const int xbl = a.W / WG_KB;
 
+    // k-block index = (image * xbl + segment) * H + row; both roles walk the columns alike
     if (warp == 0) {
         // ------------------------------------------------------------ TMA
         if (lane == 0) {
@@ -860,117 +880,89 @@ __global__ void __launch_bounds__(WG_THREADS, 1)
             const CUtensorMap *mx = ch < a.C0 ? &mx0 : &mx1;
             const int chx = ch < a.C0 ? ch : ch - a.C0;
             bool ok = true;
-            int g = 0;
-            for (; g < nk && ok; ++g) {
-                const int s = g % STS;
-                const uint32_t u = (uint32_t)(g / STS);
-                if (u >= 1 && !(ok = tc_wait(&sfree[s], (u - 1) & 1, abort_flag, a.err))) break;
-                const long long kb = kb0 + g;
-                const int xb = (int)(kb % xbl);
-                const long long r = kb / xbl;
-                const int y = (int)(r % a.H), n = (int)(r / a.H), x0 = xb * WG_KB;
-                // slot: the dY box(es) first (1024-byte aligned, as the 128-byte
-                // swizzle needs), then the three input row boxes (512-byte aligned)
-                uint8_t *st = stg + s * STG;
-                mbar_arrive_expect_tx(&full[s], TX);
-                if (BN == 32) {
-                    tma_load_4d(st, &mdy, 0, x0, y, n, &full[s]);
-                } else {
-                    for (int b = 0; b < BN / 64; ++b)
-                        tma_load_4d(st + b * WG_KB * 128, &mdy, 64 * b, x0, y, n, &full[s]);
+            uint32_t r = 0;                                    // slots loaded
+            for (long long kb = kb0; kb < kb1 && ok;) {
+                const int y0 = (int)(kb % a.H);
+                const long long col = kb / a.H;
+                const int x0 = (int)(col % xbl) * WG_KB, n = (int)(col / xbl);
+                const int cnt = kb1 - kb < a.H - y0 ? (int)(kb1 - kb) : a.H - y0;
+                for (int y = y0 - 1; y <= y0 + cnt; ++y, ++r) {
+                    const uint32_t s = r % RS, u = r / RS;
+                    if (u >= 1 && !(ok = tc_wait(&sfree[s], (u - 1) & 1, abort_flag, a.err))) break;
+                    uint8_t *st = ring + s * SLOT;
+                    mbar_arrive_expect_tx(&full[s], SLOT);
+                    for (int kx = 0; kx < 3; ++kx)
+                        tma_load_4d(st + kx * WG9_X, mx, chx, x0 + kx - 1, y, n, &full[s]);
+                    if (BN == 32) {
+                        tma_load_4d(st + 3 * WG9_X, &mdy, 0, x0, y, n, &full[s]);
+                    } else {
+                        for (int b = 0; b < BN / 64; ++b)
+                            tma_load_4d(st + 3 * WG9_X + b * WG_KB * 128, &mdy, 64 * b, x0, y, n, &full[s]);
+                    }
                 }
-                for (int ky = 0; ky < 3; ++ky)
-                    tma_load_4d(st + WG_KB * BN * 2 + ky * WG9_BOXB, mx, chx, x0 - 1, y + ky - 1, n, &full[s]);
+                kb += cnt;
             }
-            for (int s = 0; s < STS && s < g; ++s)
-                mbar_wait_bounded(&full[s], (uint32_t)((g - 1 - s) / STS) & 1, TC_WAIT_LIMIT);
+            // whatever was issued has landed before the block may end
+            for (uint32_t s = 0; s < RS && s < r; ++s)
+                mbar_wait_bounded(&full[s], ((r - 1 - s) / RS) & 1, TC_WAIT_LIMIT);
         }
         __syncwarp();
     } else if (warp == 1) {
         // ------------------------------------------------------------ MMA
         if (lane == 0) {
             bool ok = true;
-            for (int g = 0; g < nk && ok; ++g) {
-                const int s = g % STO;
-                const uint32_t u = (uint32_t)(g / STO);
-                if (!(ok = tc_wait(&opfull[s], u & 1, abort_flag, a.err))) break;
-                tc_fence_after();
-                const uint32_t sb = smem_u32(ops + s * OPS), sa = sb + BN * 128;
-                const uint64_t bd = umma_desc(sb, 1024, 2);
+            uint32_t r = 0, landed = 0;                        // first slot of the k-block, slots waited for
+            uint32_t first = 0;                                // 0 on the very first k-block
+            for (long long kb = kb0; kb < kb1 && ok;) {
+                const int y0 = (int)(kb % a.H);
+                const int cnt = kb1 - kb < a.H - y0 ? (int)(kb1 - kb) : a.H - y0;
+                for (int i = 0; i < cnt && ok; ++i, ++r) {
+                    for (; landed < r + 3 && ok; ++landed)
+                        ok = tc_wait(&full[landed % RS], (landed / RS) & 1, abort_flag, a.err);
+                    if (!ok) break;
+                    tc_fence_after();
+                    const uint32_t base = smem_u32(ring);
+                    const uint64_t bd = umma_desc_mn(base + ((r + 1) % RS) * SLOT + 3 * WG9_X, B_LBO, B_SBO, B_LAYOUT);
 #pragma unroll
-                for (int mb = 0; mb < 3; ++mb) {
-                    const uint64_t ad = umma_desc(sa + (uint32_t)(mb * 128 * 128), 1024, 2);
+                    for (int ky = 0; ky < 3; ++ky) {
+                        const uint64_t ad = umma_desc_mn(base + ((r + ky) % RS) * SLOT, WG9_X, 512, 4);
 #pragma unroll
-                    for (int j = 0; j < WG_KB / 16; ++j)
-                        tc_mma(tmem + (uint32_t)(mb * BN), ad + (uint64_t)(2 * j), bd + (uint64_t)(2 * j), IDESC,
-                               (g | j) != 0);
+                        for (int j = 0; j < WG_KB / 16; ++j)   // 16 pixels: two groups of eight
+                            tc_mma(tmem + (uint32_t)(ky * BN), ad + (uint64_t)(j * 2 * 512 / 16),
+                                   bd + (uint64_t)(j * 2 * B_SBO / 16), IDESC, first | (uint32_t)j);
+                    }
+                    first = 1;
+                    tc_commit(&sfree[r % RS]);
                 }
-                tc_commit(&opfree[s]);
+                if (ok) {                                      // the column's last two slots
+                    tc_commit(&sfree[r % RS]);
+                    tc_commit(&sfree[(r + 1) % RS]);
+                    r += 2;
+                }
+                kb += cnt;
             }
             if (ok) tc_commit(accf);
             tc_commit(drain);
             mbar_wait_bounded(drain, 0, TC_WAIT_LIMIT);
         }
         __syncwarp();
-    } else {
-        // ------------------------------------------------- transpose, epilogue
-        const int tw = warp - 2, j = lane >> 3, i = lane & 7;
-        bool ok = true;
-        for (int g = 0; g < nk && ok; ++g) {
-            const int ss = g % STS, so = g % STO;
-            if (!(ok = tc_wait(&full[ss], (uint32_t)(g / STS) & 1, abort_flag, a.err))) break;
-            if (g >= STO && !(ok = tc_wait(&opfree[so], (uint32_t)(g / STO - 1) & 1, abort_flag, a.err))) break;
-            const uint32_t sy = smem_u32(stg + ss * STG), sx = sy + WG_KB * BN * 2;
-            const uint32_t opB = smem_u32(ops + so * OPS), opA = opB + BN * 128;
-            uint32_t r[4];
-            // A: op o -> tap o / 8, pixels 8 (o % 8) ..; tap (ky, kx) reads box ky at
-            // pixel offset kx (the box starts one pixel left of x0); 64-byte rows,
-            // 16-byte chunk k of row p at (k ^ ((p >> 1) & 3))
-#pragma unroll 2
-            for (int o = tw; o < 72; o += 4) {
-                const int tap = o >> 3, k = o & 7, ky = tap / 3, kx = tap - 3 * ky;
-                const int p = 8 * k + i + kx;
-                ldsm_x4_trans(sx + ky * WG9_BOXB + p * 64 + ((j ^ ((p >> 1) & 3)) << 4), r);
-                const int row = 32 * tap + 8 * j + i;
-                stsm_x4(opA + row * 128 + ((k ^ (row & 7)) << 4), r);
-            }
+    } else if (kb1 > kb0 && wg9_wait_all(accf, kb1 - kb0, abort_flag, a.err)) {
+        // ------------------------------------------------------- epilogue
+        tc_fence_after();
+        const int q = warp & 3, kx = q;                        // rows 32 q ..: shift kx; q = 3 is the unused block
+        if (kx < 3) {
 #pragma unroll 1
-            for (int o = tw; o < BN / 4; o += 4) {
-                const int pb = o & 7, cb = 4 * (o >> 3) + j, px = 8 * pb + i;
-                uint32_t src;
-                if (BN == 32) src = sy + px * 64 + ((cb ^ ((px >> 1) & 3)) << 4);
-                else src = sy + (cb >> 3) * (WG_KB * 128) + px * 128 + (((cb & 7) ^ (px & 7)) << 4);
-                ldsm_x4_trans(src, r);
-                const int row = 8 * cb + i;
-                stsm_x4(opB + row * 128 + ((pb ^ (row & 7)) << 4), r);
-            }
-            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-            __syncwarp();
-            if (lane == 0) {
-                mbar_arrive(&sfree[ss]);
-                mbar_arrive(&opfull[so]);
-            }
-        }
-        if (ok && nk > 0 && tc_wait(accf, 0, abort_flag, a.err)) {
-            tc_fence_after();
-            const int q = warp & 3;
-#pragma unroll 1
-            for (int mb = 0; mb < 3; ++mb) {
-                const int row = mb * 128 + 32 * q + lane;      // tap * 32 + channel of the chunk
-                const bool valid = row < 288;
-                const int rg = (row >> 5) * Cin + cc * 32 + (row & 31);
-                float *dst = a.part + ((size_t)split * 9 * Cin + (valid ? rg : 0)) * BN;
+            for (int ky = 0; ky < 3; ++ky) {
+                float *dst = a.part + ((size_t)split * 9 * Cin + (3 * ky + kx) * Cin + cc * 32 + lane) * BN;
 #pragma unroll 1
                 for (int c = 0; c < BN / 32; ++c) {
                     uint32_t v[32];
-                    tmem_ld32(tmem + ((uint32_t)(32 * q) << 16) + (uint32_t)(mb * BN + 32 * c), v);
-                    if (valid) {
+                    tmem_ld32(tmem + ((uint32_t)(32 * q) << 16) + (uint32_t)(ky * BN + 32 * c), v);
 #pragma unroll
-                        for (int e = 0; e < 32; e += 4)
-                            *reinterpret_cast<float4 *>(dst + 32 * c + e) =
-                                make_float4(__uint_as_float(v[e]), __uint_as_float(v[e + 1]),
-                                            __uint_as_float(v[e + 2]), __uint_as_float(v[e + 3]));
-                    }
+                    for (int e = 0; e < 32; e += 4)
+                        *reinterpret_cast<float4 *>(dst + 32 * c + e) =
+                            make_float4(__uint_as_float(v[e]), __uint_as_float(v[e + 1]), __uint_as_float(v[e + 2]),
+                                        __uint_as_float(v[e + 3]));
                 }
             }
         }
@@ -983,24 +975,21 @@ __global__ void __launch_bounds__(WG_THREADS, 1)
     }
 }
 
+// slots that fit beside the barriers, at most twelve
 template <int BN>
-constexpr int wg9_stages_stg()
+constexpr int wg9_slots()
 {
-    return (int)((224 * 1024 - 2 * wg9_op_bytes<BN>() - WG9_SLACK - 1280) / wg9_stg_bytes<BN>()) > 8
-               ? 8
-               : (int)((224 * 1024 - 2 * wg9_op_bytes<BN>() - WG9_SLACK - 1280) / wg9_stg_bytes<BN>());
+    return (226 * 1024 - 1280) / wg9_slot_bytes<BN>() > 12 ? 12 : (226 * 1024 - 1280) / wg9_slot_bytes<BN>();
 }
 
 template <int BN>
 int launch_wgrad_tc9(const CUtensorMap &m0, const CUtensorMap &m1, const CUtensorMap &mdy, const WgTcArgs &a,
                      int ctas, cudaStream_t st)
 {
-    constexpr int STO = 2, STS = wg9_stages_stg<BN>();
-    static_assert(STS >= 2, "staging ring");
-    constexpr size_t SMEM = (size_t)STS * wg9_stg_bytes<BN>() + (size_t)STO * wg9_op_bytes<BN>() + WG9_SLACK +
-                            1024 + 256;
+    constexpr int RS = wg9_slots<BN>();
+    constexpr size_t SMEM = (size_t)RS * wg9_slot_bytes<BN>() + 1024 + 256;
     static_assert(SMEM <= 227 * 1024, "shared memory");
-    auto kern = wgrad_tc9_kernel<BN, STS, STO>;
+    auto kern = wgrad_tc9_kernel<BN, RS>;
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM) != cudaSuccess) return 1;
     count_launch();
     kern<<<ctas, WG_THREADS, SMEM, st>>>(m0, m1, mdy, a);
@@ -1152,13 +1141,13 @@ int launch_wgrad_tc(const CUtensorMap &m0, const CUtensorMap &m1, const CUtensor
 
 // Tensor map of an NHWC activation for the weight gradient: boxes of
 // (bc channels, 64 pixels, 1 row, 1 image), 64-byte (bc 32) or 128-byte (bc 64) swizzled rows.
-bool encode_wg(CUtensorMap *m, const void *ptr, int C, int N, int H, int W, int bc, int bw = WG_KB)
+bool encode_wg(CUtensorMap *m, const void *ptr, int C, int N, int H, int W, int bc)
 {
     EncodeTiledFn enc = encode_fn();
     if (!enc) return false;
     cuuint64_t dims[4] = {(cuuint64_t)C, (cuuint64_t)W, (cuuint64_t)H, (cuuint64_t)N};
     cuuint64_t strides[3] = {(cuuint64_t)C * 2, (cuuint64_t)W * C * 2, (cuuint64_t)H * W * C * 2};
-    cuuint32_t box[4] = {(cuuint32_t)bc, (cuuint32_t)bw, 1, 1};
+    cuuint32_t box[4] = {(cuuint32_t)bc, (cuuint32_t)WG_KB, 1, 1};
     cuuint32_t es[4] = {1, 1, 1, 1};
     return enc(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void *>(ptr), dims, strides, box, es,
                CU_TENSOR_MAP_INTERLEAVE_NONE, bc == 64 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B,
@@ -1287,8 +1276,8 @@ int conv3x3_wgrad_tc(const void *dy, const void *x0, int C0, const void *x1, int
     if (C0 % 32 || C1 % 32 || C0 <= 0 || W % WG_KB || N < 1 || H < 1) return 2;
     if (!(Cout == 32 || Cout == 64 || Cout == 128 || Cout == 256)) return 2;
     const int Cin = C0 + C1;
-    // Cout <= 128: all nine taps per CTA (one 32-channel input chunk, inputs
-    // staged once per k-block); Cout = 256: 128-row blocks of (tap, channel)
+    // Cout <= 128: all nine taps per CTA (one 32-channel input chunk,
+    // operands used as they land); Cout = 256: 128-row blocks of (tap, channel)
     // (three accumulators of 256 columns would not fit TMEM)
     const bool nine = Cout <= 128 && g_wgrad_nine;
     WgTcArgs a;
@@ -1322,10 +1311,9 @@ int conv3x3_wgrad_tc(const void *dy, const void *x0, int C0, const void *x1, int
     if (!ws) return 1;
     a.part = ws;
     CUtensorMap m0, m1, mdy;
-    const int bw = nine ? WG9_BOX : WG_KB;
-    if (!encode_wg(&m0, x0, C0, N, H, W, 32, bw)) return 2;
+    if (!encode_wg(&m0, x0, C0, N, H, W, 32)) return 2;
     if (C1 > 0) {
-        if (!encode_wg(&m1, x1, C1, N, H, W, 32, bw)) return 2;
+        if (!encode_wg(&m1, x1, C1, N, H, W, 32)) return 2;
     } else {
         m1 = m0;
     }

@@ -35,7 +35,13 @@ def test_halo_tiles(oracle, N, H, W, Cin, Co, split):
     assert rel_l2(_f64(y), _f64(tap)) <= 2e-3, rel_l2(_f64(y), _f64(tap))
 
 
-@pytest.mark.parametrize("N,H,W,Cin,Co", [(1, 1, 64, 32, 32), (1, 24, 64, 64, 64), (1, 40, 64, 96, 32), (1, 16, 128, 32, 256)])
+@pytest.mark.parametrize("N,H,W,Cin,Co", [
+    (1, 1, 64, 32, 32), (1, 24, 64, 64, 64), (1, 40, 64, 96, 32), (1, 16, 128, 32, 256),
+    (9, 1, 64, 32, 32),         # columns of one row: three ring slots per k-block
+    (3, 13, 128, 64, 64),       # ranges that start and end inside a column and span several
+    (1, 700, 64, 1024, 128),    # long columns: the ring goes round
+    (40, 37, 64, 32, 32),
+])
 def test_wgrad_splits(oracle, N, H, W, Cin, Co):
     import torch
     from sscRaft import warmstart as ws
