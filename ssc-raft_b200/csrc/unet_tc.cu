@@ -96,6 +96,35 @@ __device__ __forceinline__ void tc_mma(uint32_t d_tmem, uint64_t adesc, uint64_t
         : "memory");
 }
 
+// The same two, executed by a whole converged warp with warp-uniform operands and
+// issued by its elected lane.
+__device__ __forceinline__ uint32_t elect_one()
+{
+    uint32_t e;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(e));
+    return e;
+}
+__device__ __forceinline__ void tc_mma_if(uint32_t go, uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
+                                          uint32_t acc)
+{
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "setp.ne.b32 q, %5, 0;\n\t"
+        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
+        "l"(adesc), "l"(bdesc), "r"(idesc), "r"(acc), "r"(go)
+        : "memory");
+}
+__device__ __forceinline__ void tc_commit_if(uint32_t go, uint64_t *bar)
+{
+    asm volatile("{\n\t.reg .pred q;\n\t"
+                 "setp.ne.b32 q, %1, 0;\n\t"
+                 "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(
+                     smem_u32(bar)),
+                 "r"(go)
+                 : "memory");
+}
+
 // 32 consecutive 32-bit TMEM columns of this thread's lane
 __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32])
 {
@@ -532,7 +561,7 @@ bool encode_w(CUtensorMap *m, const void *ptr, int Cout, int Cin, int KC, int BN
                CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-bool g_halo = true;   // halo tiles for the 32 -> 32 channel layers (raft_unet_set_conv_halo)
+bool g_halo = true;   // halo tiles for layers with few channels (raft_unet_set_conv_halo)
 bool g_wgrad_nine = true;   // nine-tap weight-gradient CTAs where Cout <= 128 (raft_unet_set_wgrad_nine)
 
 // =========================================================== weight gradient
@@ -787,11 +816,14 @@ __global__ void __launch_bounds__(WG_THREADS, 1)
 // 128 rows = the three shifts of slot y + ky - 1 and, as the unused fourth block of
 // 32, the first 4 KB of that slot's dY: 96 of its 128 accumulator rows are read.
 // Transposing each k-block into K-major operands with ldmatrix / stmatrix had four
-// warps moving 73 KB per k-block.  Bound by the MMA reading 128 x 16 input operands
-// with 64-byte rows, about 120 clocks each (input loaded once with taps as row
-// offsets instead of three times: no change).  Kernel alone before, with the
-// 10 - 15 us reduction after: 8 x 512^2, 32 -> 32: 242 -> 184 us; 96 -> 32: 713 ->
-// 490 us; 8 x 256^2, 192 -> 64: 405 -> 272 us; 8 x 128^2, 384 -> 128: 253 -> 155 us.
+// warps moving 73 KB per k-block.  The MMA warp runs converged and its elected
+// lane issues: from one lane of a divergent branch an issue took about 120 clocks
+// (descriptors in per-thread registers), whatever the operands; the input loaded
+// once with taps as row offsets, or the operands' roles exchanged, changed nothing.
+// Kernel alone at first, then with the 10 - 15 us reduction untransposed and with
+// the converged issue: 8 x 512^2, 32 -> 32: 242, 183, 120 us; 96 -> 32: 713, 489,
+// 296 us; 8 x 256^2, 192 -> 64: 405, 266, 186 us; 8 x 128^2, 384 -> 128: 253, 158,
+// 130 us.
 constexpr int WG9_X = WG_KB * 64;             // one shifted copy: 64 pixels x 32 channels
 
 template <int BN>
@@ -909,7 +941,9 @@ __global__ void __launch_bounds__(WG_THREADS, 1)
         __syncwarp();
     } else if (warp == 1) {
         // ------------------------------------------------------------ MMA
-        if (lane == 0) {
+        {
+            // the whole warp walks along, so that the operands stay warp-uniform
+            const uint32_t go = elect_one();
             bool ok = true;
             uint32_t r = 0, landed = 0;                        // first slot of the k-block, slots waited for
             uint32_t first = 0;                                // 0 on the very first k-block
@@ -918,7 +952,8 @@ __global__ void __launch_bounds__(WG_THREADS, 1)
                 const int cnt = kb1 - kb < a.H - y0 ? (int)(kb1 - kb) : a.H - y0;
                 for (int i = 0; i < cnt && ok; ++i, ++r) {
                     for (; landed < r + 3 && ok; ++landed)
-                        ok = tc_wait(&full[landed % RS], (landed / RS) & 1, abort_flag, a.err);
+                        ok = __all_sync(0xffffffffu,
+                                        tc_wait(&full[landed % RS], (landed / RS) & 1, abort_flag, a.err));
                     if (!ok) break;
                     tc_fence_after();
                     const uint32_t base = smem_u32(ring);
@@ -928,21 +963,21 @@ __global__ void __launch_bounds__(WG_THREADS, 1)
                         const uint64_t ad = umma_desc_mn(base + ((r + ky) % RS) * SLOT, WG9_X, 512, 4);
 #pragma unroll
                         for (int j = 0; j < WG_KB / 16; ++j)   // 16 pixels: two groups of eight
-                            tc_mma(tmem + (uint32_t)(ky * BN), ad + (uint64_t)(j * 2 * 512 / 16),
+                            tc_mma_if(go, tmem + (uint32_t)(ky * BN), ad + (uint64_t)(j * 2 * 512 / 16),
                                    bd + (uint64_t)(j * 2 * B_SBO / 16), IDESC, first | (uint32_t)j);
                     }
                     first = 1;
-                    tc_commit(&sfree[r % RS]);
+                    tc_commit_if(go, &sfree[r % RS]);
                 }
                 if (ok) {                                      // the column's last two slots
-                    tc_commit(&sfree[r % RS]);
-                    tc_commit(&sfree[(r + 1) % RS]);
+                    tc_commit_if(go, &sfree[r % RS]);
+                    tc_commit_if(go, &sfree[(r + 1) % RS]);
                     r += 2;
                 }
                 kb += cnt;
             }
-            if (ok) tc_commit(accf);
-            tc_commit(drain);
+            if (ok) tc_commit_if(go, accf);
+            tc_commit_if(go, drain);
             mbar_wait_bounded(drain, 0, TC_WAIT_LIMIT);
         }
         __syncwarp();
