@@ -36,10 +36,6 @@ sys.path.insert(0, os.path.join(REPO, "ssc-raft_b200"))
 N_RAYS, N_ANGLES, N_SLICES = 2048, 1800, 512
 OFFSET, PAD, FILTER_ID = 3.5, 2, 5          # Hann
 I0 = 1.0e4
-# DRAM bytes (read + write) of one 32-slice nearest backprojector launch at
-# 2048^2 x 1800 angles (four slices per CTA on slice-interleaved rows),
-# measured with ncu (1.08x the algorithmic bytes).
-BP_TRAFFIC_PER_LAUNCH = 783_763_456 + 518_802_944
 WORKLOAD = ("batched FBP: 512 slices x 2048^2, 1800 angles over [0,pi), 2048 bins, "
             "axis offset +3.5 px, Hann, padding 2")
 METRIC = "FBP slices/s at 2048^2 x 1800 angles"
@@ -947,7 +943,7 @@ def run_ours(args):
     sm_mhz = (clocks or {}).get("sm_mhz") or sm_max
     gups_bp = upd_per_launch / bp_avg_s / 1e9
     peak_gups = gather_peak_gups(4, 4, sm_mhz)
-    # f32 pairs: 8 B + 5 FP32 ops per update; bf16 pairs on slice-interleaved rows:
+    # linear f32: two samples, 8 B + 5 FP32 ops per update; bf16 pairs on slice-interleaved rows:
     # 4 B + 4 ops (two FP32, two integer to unpack the pair)
     for name, (g, s, bytes_upd, ops) in (("linear_fp32", (1, 1, 8, 5)), ("linear_bf16", (1, 2, 4, 4))):
         _, _, vms, vn = profile_bp(g, s)
@@ -994,15 +990,15 @@ def run_ours(args):
                     "max_abs_diff_vs_device_path": spot},
             "roofline": {"bound": "smem-gather", "achieved": gups_bp, "peak": peak_gups, "unit": "GUPS",
                          "frac": gups_bp / peak_gups,
-                         "kernel": "bp_kernel_s4<nearest,f32,interleaved>",
+                         "kernel": "bp_run_kernel<nearest,f32,16 slices per thread>",
                          "kernel_ms_per_launch": bp_avg_s * 1e3,
                          "updates_per_launch": upd_per_launch,
                          "peak_def": "148 SMs x SM clock (median sampled) x 32 updates/clk: 128 B/clk of "
-                                     "shared-memory data pipe / 4 B per update",
+                                     "shared-memory data pipe / 4 B per update (one sample read per update; "
+                                     "the run kernel reads 2.6 B, so frac can pass 1)",
                          "sm_mhz": sm_mhz,
-                         "traffic": BP_TRAFFIC_PER_LAUNCH if chunk == 32 else None,
-                         "traffic_source": "ncu dram__bytes_read.sum + dram__bytes_write.sum of one 32-slice "
-                                           "launch (S4 interleaved, AB16), --set full capture",
+                         "traffic": None,
+                         "traffic_source": "not captured at this size",
                          "algorithmic_bytes_per_launch": alg_bytes,
                          "hbm": {"achieved_gbs": alg_bytes / bp_avg_s / 1e9, "peak_gbs": hbm_peak,
                                  "frac": alg_bytes / bp_avg_s / 1e9 / hbm_peak, "peak_kind": peak_kind}},
