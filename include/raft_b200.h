@@ -281,12 +281,14 @@ int raft_unet_set_conv_path(int path);
 int raft_unet_set_conv_halo(int on);
 /* tcgen05 weight gradient (W a multiple of 64; Cout 32, 64, 128 or 256; other shapes and
  * raft_unet_set_conv_path(1) use the mma.sync kernel): 1 = for Cout <= 128 one CTA per
- * 32-channel input chunk with all nine taps, the input staged once per 64-pixel k-block
- * (default); 0 = 128-row blocks of (tap, channel) for every layer. */
+ * 32-channel input chunk with all nine taps (default); 0 = 128-row blocks of (tap, channel)
+ * for every layer. */
 int raft_unet_set_wgrad_nine(int on);
 /* 1 if a bounded pipeline wait of the tcgen05 convolution ran out since the last call
  * (the flag is then cleared); synchronises the current device. */
 int raft_unet_conv_error(void);
+/* Partial sums of raft_unet_conv_wgrad and raft_unet_relu_bwd_bias live in stream-ordered
+ * memory of the call's own: calls on several streams and threads do not share any. */
 int raft_unet_conv_wgrad(const void *dy, const void *x0, int C0, const void *x1, int C1, float *dw,
                          float *dbias, int N, int H, int W, int Cout, void *stream);
 int raft_unet_flip_weights(const void *w, void *wt, int Cout, int Cin, void *stream);
@@ -295,6 +297,14 @@ int raft_unet_relu_bwd(const void *y, const void *dy, void *dpre, size_t n, void
  * dpre, in a fixed order.  C a power of two from 8 to 256, 16-byte aligned tensors. */
 int raft_unet_relu_bwd_bias(const void *y, const void *dy, void *dpre, float *dbias, size_t pixels, int C,
                             void *stream);
+/* raft_unet_relu_bwd, the bias gradient and raft_unet_conv_wgrad of one layer: dpre = dy where
+ * y > 0, dbias += its sums, dw += its weight gradient (arguments as above).  work holds
+ * work_floats >= raft_unet_layer_grads_work(C0 + C1, Cout) floats of the caller's for the
+ * partial sums, used in stream order; with NULL the call takes its own. */
+size_t raft_unet_layer_grads_work(int Cin, int Cout);
+int raft_unet_layer_grads(const void *y, const void *dy, void *dpre, const void *x0, int C0, const void *x1,
+                          int C1, float *dw, float *dbias, int N, int H, int W, int Cout, float *work,
+                          size_t work_floats, void *stream);
 int raft_unet_pool(int backward, const void *src, void *dst, int N, int H, int W, int C, void *stream);
 int raft_unet_upsample(int backward, const void *src, void *dst, int N, int H, int W, int C, void *stream);
 int raft_unet_input(const float *img, const float *scale, void *x, int N, int H, int W, int C, void *stream);

@@ -355,11 +355,15 @@ int conv3x3_tc(const void *x0, int C0, const void *x1, int C1, const void *w, co
 int conv3x3_tc_error();
 // Weight (and bias) gradient of the 3x3 convolution on tcgen05 (unet_tc.cu);
 // 0 = launched, 1 = launch error, 2 = shape not handled (W % 64, Cout not 32/64/128/256).
+// work: conv3x3_wgrad_work floats for the partial sums, or null (stream-ordered memory).
 int conv3x3_wgrad_tc(const void *dy, const void *x0, int C0, const void *x1, int C1, float *dw, float *dbias, int N,
-                     int H, int W, int Cout, cudaStream_t st);
+                     int H, int W, int Cout, float *work, size_t work_floats, cudaStream_t st);
+bool conv3x3_wgrad_tc_supported(int C0, int C1, int N, int H, int W, int Cout);
+size_t conv3x3_wgrad_work(int Cin, int Cout);
 void conv3x3_wgrad_tc_set_nine(int on);
-// ReLU backward with the bias gradient (unet_tc.cu); 0 = launched, 1 = error.
-int relu_bwd_bias(const void *y, const void *dy, void *dpre, float *dbias, long long P, int C, cudaStream_t st);
+// ReLU backward with the bias gradient (unet_tc.cu; work as above); 0 = launched, 1 = error.
+int relu_bwd_bias(const void *y, const void *dy, void *dpre, float *dbias, long long P, int C, float *work,
+                  size_t work_floats, cudaStream_t st);
 void conv3x3_tc_set_halo(int on);
 
 }  // namespace raft

@@ -1178,28 +1178,65 @@ bool encode_wg(CUtensorMap *m, const void *ptr, int C, int N, int H, int W, int 
                CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-// Grow-only per-device workspace of the weight gradient's partial sums.
-float *wgrad_workspace(int device, size_t floats)
-{
-    static std::mutex mu;
-    static float *buf[64] = {};
-    static size_t cap[64] = {};
-    std::lock_guard<std::mutex> lk(mu);
-    if (device < 0 || device >= 64) return nullptr;
-    if (cap[device] < floats) {
-        if (buf[device]) cudaFree(buf[device]);
-        buf[device] = nullptr;
-        cap[device] = 0;
-        if (cudaMalloc(&buf[device], floats * sizeof(float)) != cudaSuccess) return nullptr;
-        cap[device] = floats;
+// Partial sums of one gradient: the caller's memory, or stream-ordered memory for the
+// time of the launches.  Never shared between calls: calls on other streams or
+// threads may run at the same time.
+struct Partials {
+    float *p = nullptr;
+    bool own = false;
+    cudaStream_t st;
+    Partials(float *work, size_t have, size_t need, cudaStream_t stream) : st(stream)
+    {
+        if (work) {
+            if (have >= need) p = work;
+            return;
+        }
+        if (cudaMallocAsync((void **)&p, need * sizeof(float), st) == cudaSuccess) own = true;
+        else p = nullptr;
     }
-    return buf[device];
+    ~Partials()
+    {
+        if (own) cudaFreeAsync(p, st);
+    }
+    Partials(const Partials &) = delete;
+    Partials &operator=(const Partials &) = delete;
+};
+
+int sm_count()
+{
+    int dev = 0, sms = 148;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    return sms;
 }
+
+// Pixel ranges of the weight gradient.  The largest number whose CTAs run in one
+// wave: shared memory holds one CTA per SM (164-224 KB), and a CTA past the last SM
+// doubles the launch (96 -> 32 channels at 8 x 512^2: 1327 us with 150 CTAs).
+long long wgrad_splits(int sms, int items) { return std::max(1, sms / items); }
+int wgrad_items(bool nine, int Cin) { return nine ? Cin / 32 : (9 * Cin / 32 + 3) / 4; }
+int wgrad_rows(bool nine, int Cin) { return nine ? 9 * Cin : wgrad_items(false, Cin) * 128; }
 
 }  // namespace
 
 void conv3x3_tc_set_halo(int on) { g_halo = on != 0; }
 void conv3x3_wgrad_tc_set_nine(int on) { g_wgrad_nine = on != 0; }
+
+bool conv3x3_wgrad_tc_supported(int C0, int C1, int N, int H, int W, int Cout)
+{
+    if (C0 % 32 || C1 % 32 || C0 <= 0 || W % WG_KB || N < 1 || H < 1) return false;
+    return Cout == 32 || Cout == 64 || Cout == 128 || Cout == 256;
+}
+
+// Floats of partial sums that the gradients of a Cin -> Cout layer take at most.
+size_t conv3x3_wgrad_work(int Cin, int Cout)
+{
+    const int sms = sm_count();
+    size_t n = 0;
+    for (bool nine : {false, true})
+        n = std::max(n, (size_t)wgrad_splits(sms, wgrad_items(nine, Cin)) * wgrad_rows(nine, Cin) * Cout);
+    return n + (size_t)4 * sms * Cout;
+}
 
 bool conv3x3_tc_supported(int C0, int C1, int W)
 {
@@ -1294,11 +1331,11 @@ int conv3x3_tc(const void *x0, int C0, const void *x1, int C1, const void *w, co
 }
 
 // 0 = launched, 1 = launch error, 2 = shape not handled here (caller uses the mma.sync kernel)
+// work: conv3x3_wgrad_work floats, or null (stream-ordered memory of the call's own)
 int conv3x3_wgrad_tc(const void *dy, const void *x0, int C0, const void *x1, int C1, float *dw, float *dbias, int N,
-                     int H, int W, int Cout, cudaStream_t st)
+                     int H, int W, int Cout, float *work, size_t work_floats, cudaStream_t st)
 {
-    if (C0 % 32 || C1 % 32 || C0 <= 0 || W % WG_KB || N < 1 || H < 1) return 2;
-    if (!(Cout == 32 || Cout == 64 || Cout == 128 || Cout == 256)) return 2;
+    if (!conv3x3_wgrad_tc_supported(C0, C1, N, H, W, Cout)) return 2;
     const int Cin = C0 + C1;
     // Cout <= 128: all nine taps per CTA (one 32-channel input chunk,
     // operands used as they land); Cout = 256: 128-row blocks of (tap, channel)
@@ -1312,28 +1349,23 @@ int conv3x3_wgrad_tc(const void *dy, const void *x0, int C0, const void *x1, int
     a.C1 = C1;
     a.Cout = Cout;
     a.nchunks = 9 * Cin / 32;
-    a.mtiles = (a.nchunks + 3) / 4;
+    a.mtiles = wgrad_items(false, Cin);
     a.kblocks = (long long)N * H * (W / WG_KB);
-    int dev = 0, sms = 148;
+    int dev = 0;
     cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    // The largest number of pixel ranges whose CTAs run in one wave: shared memory
-    // holds one CTA per SM (164-224 KB), and a CTA past the last SM doubles the
-    // launch (96 -> 32 channels at 8 x 512^2: 1327 us with 150 CTAs).  At least 8
-    // k-blocks per CTA.
-    const int items = nine ? Cin / 32 : a.mtiles;
-    long long splits = std::max(1, sms / items);
-    splits = std::min(splits, std::max(1LL, a.kblocks / 8));
+    const int sms = sm_count(), items = wgrad_items(nine, Cin);
+    // at least 8 k-blocks per CTA
+    const long long splits = std::min(wgrad_splits(sms, items), std::max(1LL, a.kblocks / 8));
     a.kper = (a.kblocks + splits - 1) / splits;
     a.splits = (int)((a.kblocks + a.kper - 1) / a.kper);
     a.err = tc_err_flag(dev);
     const long long P = (long long)N * H * W;
     const int bias_blk = dbias ? (int)std::min<long long>(4 * sms, std::max(1LL, P / 256)) : 0;
-    const int prow = nine ? 9 * Cin : a.mtiles * 128;
+    const int prow = wgrad_rows(nine, Cin);
     const size_t part_floats = (size_t)a.splits * prow * Cout;
-    float *ws = wgrad_workspace(dev, part_floats + (size_t)bias_blk * Cout);
-    if (!ws) return 1;
-    a.part = ws;
+    const Partials ws(work, work_floats, part_floats + (size_t)bias_blk * Cout, st);
+    if (!ws.p) return 1;
+    a.part = ws.p;
     CUtensorMap m0, m1, mdy;
     if (!encode_wg(&m0, x0, C0, N, H, W, 32)) return 2;
     if (C1 > 0) {
@@ -1364,7 +1396,7 @@ int conv3x3_wgrad_tc(const void *dy, const void *x0, int C0, const void *x1, int
     wgrad_reduce_kernel<<<dim3((rows + 3) / 4, Cout / 32), 256, 0, st>>>(a.part, dw, a.splits, rows, prow, Cout);
     if (cudaGetLastError() != cudaSuccess) return 1;
     if (dbias) {
-        float *bp = ws + part_floats;
+        float *bp = ws.p + part_floats;
         const long long per = (P + bias_blk - 1) / bias_blk;
         count_launch();
         bias_partial_kernel<<<bias_blk, 256, 0, st>>>((const bf16 *)dy, bp, P, Cout, per);
@@ -1375,14 +1407,13 @@ int conv3x3_wgrad_tc(const void *dy, const void *x0, int C0, const void *x1, int
     return 0;
 }
 
-int relu_bwd_bias(const void *y, const void *dy, void *dpre, float *dbias, long long P, int C, cudaStream_t st)
+int relu_bwd_bias(const void *y, const void *dy, void *dpre, float *dbias, long long P, int C, float *work,
+                  size_t work_floats, cudaStream_t st)
 {
     if (P < 1 || C < 8 || C > 256 || 256 % C || (((uintptr_t)y | (uintptr_t)dy | (uintptr_t)dpre) & 15)) return 1;
-    int dev = 0, sms = 148;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    const int blk = (int)std::min<long long>(4 * sms, std::max(1LL, P / 256));
-    float *part = wgrad_workspace(dev, (size_t)blk * C);
+    const int blk = (int)std::min<long long>(4 * sm_count(), std::max(1LL, P / 256));
+    const Partials ws(work, work_floats, (size_t)blk * C, st);
+    float *part = ws.p;
     if (!part) return 1;
     count_launch();
     relu_bwd_bias_kernel<<<blk, 256, 0, st>>>((const bf16 *)y, (const bf16 *)dy, (bf16 *)dpre, part, P, C,

@@ -28,6 +28,9 @@ libraft.raft_unet_conv_wgrad.argtypes = [_P, _P, _I, _P, _I, _P, _P, _I, _I, _I,
 libraft.raft_unet_flip_weights.argtypes = [_P, _P, _I, _I, _P]
 libraft.raft_unet_relu_bwd.argtypes = [_P, _P, _P, _Z, _P]
 libraft.raft_unet_relu_bwd_bias.argtypes = [_P, _P, _P, _P, _Z, _I, _P]
+libraft.raft_unet_layer_grads_work.argtypes = [_I, _I]
+libraft.raft_unet_layer_grads_work.restype = _Z
+libraft.raft_unet_layer_grads.argtypes = [_P, _P, _P, _P, _I, _P, _I, _P, _P, _I, _I, _I, _I, _P, _Z, _P]
 libraft.raft_unet_pool.argtypes = [_I, _P, _P, _I, _I, _I, _I, _P]
 libraft.raft_unet_upsample.argtypes = [_I, _P, _P, _I, _I, _I, _I, _P]
 libraft.raft_unet_input.argtypes = [_P, _P, _P, _I, _I, _I, _I, _P]
@@ -42,7 +45,7 @@ libraft.raft_unet_set_conv_path.argtypes = [_I]
 libraft.raft_unet_set_conv_halo.argtypes = [_I]
 libraft.raft_unet_set_wgrad_nine.argtypes = [_I]
 libraft.raft_unet_conv_error.argtypes = []
-for _f in ("raft_unet_set_conv_path", "raft_unet_set_conv_halo", "raft_unet_set_wgrad_nine", "raft_unet_conv_error", "raft_unet_conv_fwd", "raft_unet_conv_wgrad", "raft_unet_flip_weights", "raft_unet_relu_bwd", "raft_unet_relu_bwd_bias",
+for _f in ("raft_unet_set_conv_path", "raft_unet_set_conv_halo", "raft_unet_set_wgrad_nine", "raft_unet_conv_error", "raft_unet_conv_fwd", "raft_unet_conv_wgrad", "raft_unet_flip_weights", "raft_unet_relu_bwd", "raft_unet_relu_bwd_bias", "raft_unet_layer_grads",
            "raft_unet_pool", "raft_unet_upsample", "raft_unet_input", "raft_unet_input_conv", "raft_unet_input_wgrad",
            "raft_unet_head",
            "raft_unet_mse",
@@ -92,6 +95,7 @@ class UNet:
         self._sync_bf16()
         self.step_count = 0
         self.stream = None
+        self._part_floats = None
 
     def n_params(self):
         return sum(t.numel() for t in self.w.values()) + sum(t.numel() for t in self.b.values())
@@ -165,9 +169,9 @@ class UNet:
         _, c0, c1, co = next(l for l in self.LAYERS if l[0] == name)
         st = self._st()
         dpre = torch.empty_like(gy)
-        _ok(libraft.raft_unet_relu_bwd_bias(_p(y), _p(gy), _p(dpre), _p(self.gb[name]), N * H * W, co, st), "relu_bwd")
-        _ok(libraft.raft_unet_conv_wgrad(_p(dpre), _p(x0), c0, _p(x1), c1, _p(self.gw[name]), None,
-                                         N, H, W, co, st), "wgrad " + name)
+        _ok(libraft.raft_unet_layer_grads(_p(y), _p(gy), _p(dpre), _p(x0), c0, _p(x1), c1, _p(self.gw[name]),
+                                          _p(self.gb[name]), N, H, W, co, _p(self._part), self._part.numel(), st),
+            "grads " + name)
         if not need_dx:
             return None, None
         cin = c0 + c1
@@ -200,6 +204,12 @@ class UNet:
         self.gw = {k: torch.zeros_like(v) for k, v in self.w.items()}
         self.gb = {k: torch.zeros_like(v) for k, v in self.b.items()}
         st = self._st()
+        # the layers' partial sums, one layer after the other on this stream
+        if self._part_floats is None:
+            with torch.cuda.device(self.dev):
+                self._part_floats = max(libraft.raft_unet_layer_grads_work(c0 + c1, co)
+                                        for _, c0, c1, co in self.LAYERS)
+        self._part = torch.empty(self._part_floats, dtype=torch.float32, device=self.dev)
         g_d0 = torch.empty_like(A["d0"])
         _ok(libraft.raft_unet_head(1, _p(A["d0"]), _p(self.w["head"]), None, None, None, _p(gout), _p(g_d0),
                                    _p(self.gw["head"]), _p(self.gb["head"]), N, H * W, 32, st), "head_bwd")
@@ -229,6 +239,7 @@ class UNet:
         work = torch.empty(N * H * 320, dtype=torch.float32, device=self.dev)
         _ok(libraft.raft_unet_input_wgrad(_p(img), _p(scale), _p(dpre), _p(self.gw["e0a"]), 32, _p(self.gb["e0a"]),
                                           _p(work), work.numel(), N, H, W, st), "wgrad e0a")
+        self._part = None
 
     def adam_step(self, lr, b1=0.9, b2=0.999, eps=1e-8):
         self.step_count += 1
