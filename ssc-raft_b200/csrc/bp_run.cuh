@@ -21,6 +21,7 @@
 // conflicts): when the run axis changes, which for angles in order happens
 // twice over [0, pi), the accumulators change hands through shared memory.
 #pragma once
+#include "ring.hpp"
 
 namespace raft {
 
@@ -429,6 +430,8 @@ __global__ void __launch_bounds__(BP_THREADS, run_min_blocks(STORE, G)) bp_run_k
     constexpr int P = 4, NS = kRunStages, GW = G ? G : 1, ES = G ? 16 : 4;   // windows per angle, element bytes
     extern __shared__ __align__(128) unsigned char smem[];
     uint64_t *full = reinterpret_cast<uint64_t *>(smem), *empty = full + NS, *turned = empty + NS;
+    volatile int *armed = reinterpret_cast<volatile int *>(turned + 1);   // last stage copied into each buffer
+    using Stages = Ring<NS>;
     RunParam *prm = reinterpret_cast<RunParam *>(smem + 128);
     float *scratch = reinterpret_cast<float *>(smem + kRunFixed - kRunScratch);
     unsigned char *win = smem + kRunFixed;
@@ -442,6 +445,7 @@ __global__ void __launch_bounds__(BP_THREADS, run_min_blocks(STORE, G)) bp_run_k
         for (int i = 0; i < NS; i++) {
             mbar_init(&full[i], 1);
             mbar_init(&empty[i], BP_THREADS / 32);
+            armed[i] = -1;
         }
         mbar_init(turned, BP_THREADS / 32);
         fence_mbar_init();
@@ -449,7 +453,8 @@ __global__ void __launch_bounds__(BP_THREADS, run_min_blocks(STORE, G)) bp_run_k
     __syncthreads();
 
     // Waits are bounded; after one that ran out (reported through the error
-    // flag) the rest do not wait, so that every warp reaches the end.
+    // flag) the rest do not wait, so that every warp reaches the end, and the
+    // warp copies nothing more: the copy it waited for may still be on its way.
     bool ok = true;
     auto wait = [&](uint64_t *bar, uint32_t parity) {
         if (!mbar_wait_bounded(bar, parity, ok ? kWaitLimit : 1)) ok = false;
@@ -458,9 +463,10 @@ __global__ void __launch_bounds__(BP_THREADS, run_min_blocks(STORE, G)) bp_run_k
     // One warp: the window base and mode of every angle of stage s, then one
     // bulk copy per angle and group.  The warps take turns.
     auto issue = [&](int s) {
-        const int b = s % NS, a0 = s * AB, na = min(AB, A - a0), lane = fresh_tid() & 31;
+        const int b = Stages::buffer(s), a0 = s * AB, na = min(AB, A - a0), lane = fresh_tid() & 31;
         const int x0 = fresh_ctaid_x() * kRunTile, y0 = fresh_ctaid_y() * kRunTile;
-        if (s >= NS) wait(&empty[b], (s / NS - 1) & 1);
+        if (Stages::reused(s)) wait(&empty[b], Stages::parity(Stages::before(s)));
+        if (!__all_sync(0xffffffffu, ok)) return;
         int base = 0;
         if (lane < na) {
             AngleParam ap;
@@ -488,7 +494,10 @@ __global__ void __launch_bounds__(BP_THREADS, run_min_blocks(STORE, G)) bp_run_k
             prm[b * 32 + lane] = rp;
         }
         __syncwarp();
-        if (lane == 0) mbar_arrive_expect_tx(&full[b], (uint32_t)(na * GW * wbytes));   // releases prm
+        if (lane == 0) {
+            armed[b] = s;
+            mbar_arrive_expect_tx(&full[b], (uint32_t)(na * GW * wbytes));   // releases prm
+        }
         __syncwarp();
         if (lane < na) {
             fence_proxy_async_smem();
@@ -579,9 +588,9 @@ __global__ void __launch_bounds__(BP_THREADS, run_min_blocks(STORE, G)) bp_run_k
 
 #pragma unroll 1
     for (int s = 0; s < nst; s++) {
-        const int b = s % NS;
+        const int b = Stages::buffer(s);
         if (s + NS - 2 < nst && warp == s % (BP_THREADS / 32)) issue(s + NS - 2);
-        wait(&full[b], (s / NS) & 1);
+        wait(&full[b], Stages::parity(s));
         const int na = min(AB, A - s * AB), lane = fresh_tid() & 31;
         const unsigned char *w = win + (size_t)b * stage_bytes;
         const RunParam *pb = prm + b * 32;
@@ -611,8 +620,9 @@ __global__ void __launch_bounds__(BP_THREADS, run_min_blocks(STORE, G)) bp_run_k
     }
     if (!ok) {
         if (p.err) atomicExch(p.err, 1);
-        // give copies still in flight a last bounded chance to land
-        for (int i = 0; i < NS; i++) mbar_wait_bounded(&full[i], 1, kWaitLimit);
+        // shared memory is given back only after the copies into it have landed
+        for (int i = 0; i < NS; i++)
+            if (const int s = armed[i]; s >= 0) mbar_wait_bounded(&full[i], Stages::parity(s), kWaitLimit);
         return;
     }
 
