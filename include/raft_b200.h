@@ -247,6 +247,13 @@ int raft_slab_partition(int nslices, int ngpus, int *start, int *count);
  * geometry 0/1 with FBP packing, 2 with EM packing.  Returns 0 on success. */
 int raft_plan_window(const float *paramf, const int *parami, int geometry, int store, int *out);
 
+/* Host-only: which backprojector kernels a launch of nslices slices takes (parameters as
+ * raft_plan_window, host angles): out = {groups of four slices taken by 16, 8 and 4 slices
+ * per thread of the run kernel, groups taken by the single-pixel kernel, 1 for a single slice
+ * on plain rows by the run kernel}.  Every choice gives the same bits.  Returns 0 on success. */
+int raft_bp_split(const float *paramf, const int *parami, const float *angles, int geometry, int store,
+                  int nslices, int *out);
+
 /* sin/cos of angles[0..n) computed on `gpu` with the fast intrinsics the reference
  * uses: kind 0 = __sinf/__cosf (setSinCosTable, cuda/src/common/opt.cu:187-194),
  * kind 1 = __sincosf (kernel_backprojection, em_RT_kernel.cu:120).  Returns 0 on success. */

@@ -364,11 +364,10 @@ int raft_fbp_device(int gpu, float *d_obj, const float *d_tomogram, const float 
         FbpTables tb = fbp_tables(ds, fp, angles, st);
         const size_t tomo_ps = (size_t)cfg.nangles * cfg.nrays;
         const int chunk = std::max(1, std::min(cfg.nslices, cfg.blocksize > 0 ? cfg.blocksize : 32));
-        void *il = fbp_il_bytes(fp, chunk) ? ds.il.get(fbp_il_bytes(fp, chunk)) : nullptr;
-        void *rows = (il && fbp_fused_il(fp)) ? nullptr : ds.rows.get(fbp_rows_bytes(fp, chunk));
+        void *rows = ds.il.get(fbp_ws_bytes(fp, chunk));
         for (int s0 = 0; s0 < cfg.nslices; s0 += chunk) {
             const int ns = std::min(chunk, cfg.nslices - s0);
-            fbp_chunk(ds, fp, tb, d_tomogram + tomo_ps * s0, d_obj + (size_t)fp.No * fp.No * s0, ns, rows, st, il);
+            fbp_chunk(fp, tb, d_tomogram + tomo_ps * s0, d_obj + (size_t)fp.No * fp.No * s0, ns, rows, st, true);
         }
         if (!stream) RAFT_CUDA(cudaStreamSynchronize(st));
     } catch (const CudaFail &) {
@@ -603,6 +602,43 @@ int raft_plan_window(const float *paramf, const int *parami, int geometry, int s
     } catch (const CudaFail &) {
     }
     return has_error() ? 1 : 0;
+}
+
+// out = {groups of four slices by 16, 8 and 4 slices per thread of the run kernel, by the
+// single-pixel kernel, 1 where the one slice takes the run kernel on plain rows}
+int raft_bp_split(const float *paramf, const int *parami, const float *angles, int geometry, int store, int nslices,
+                  int *out)
+{
+    clear_error();
+    BpGeo g;
+    int No = 0, A = 0;
+    if (geometry == GEOM_EM_REF) {
+        EmConfig c;
+        if (!parse_em_arrays(paramf, parami, c)) return 1;
+        g = prepare_em(c).geo;
+        No = c.objsize;
+        A = c.nangles;
+        store = STORE_F32;
+    } else {
+        FbpConfig c;
+        if (!parse_fbp_arrays(paramf, parami, c, true) || !fbp_mode_ok(geometry, store, "raft_bp_split")) return 1;
+        g.dx = g.dt = c.pixel_x;
+        g.dy = c.pixel_y;
+        g.ratio = (double)c.pixel_y / (double)c.pixel_x;
+        No = c.objsize;
+        A = c.nangles;
+    }
+    if (!angles || !out) {
+        set_error("null data pointer");
+        return 1;
+    }
+    const BpSplit s = bp_split(g, geometry, store, No, nslices, A, bp_run_turns(angles, A));
+    out[0] = s.g16;
+    out[1] = s.g8;
+    out[2] = s.g4;
+    out[3] = s.single;
+    out[4] = s.one;
+    return 0;
 }
 
 // sin/cos of `angles` as the GPU's fast intrinsics produce them: kind 0 =

@@ -632,34 +632,6 @@ static void launch_bp_s(const BpArgs &a, int AB, cudaStream_t st)
     RAFT_CUDA(cudaGetLastError());
 }
 
-struct BpTune;
-static bool forced_tune(BpTune &t);
-
-// The run kernel: its rule on positions needs pixels as wide as detector bins.
-// Turning the accumulators costs about as much as three angles, so angle lists
-// that change the run axis more often than every 16 angles (scans in
-// golden-ratio order) keep the single-pixel kernel.  So do short nearest-sample
-// scans, whose few angles per slope class do not fill the stages: 20 x 1126^2 x 99,
-// a whole pass, 537 us with the single-pixel kernel and 656 us with runs (143 angles:
-// no slower).
-bool bp_runs_ok(const BpGeo &g, int geometry, int nangles, int turns)
-{
-    if (geometry == GEOM_FBP_REF && nangles < 128) return false;
-    if (turns > nangles / 16 + 2) return false;
-    if (geometry == GEOM_EM_REF) return g.dxy == g.dt;
-    return g.dx == g.dt && g.dy == g.dt && g.ratio == 1.0;
-}
-
-// A single slice of four-byte elements: plain rows and the one-slice form of the
-// run kernel (512^2 x 360: 50 us; 102 us when it filled a quarter of a four-slice
-// CTA).  Two and three slices of a small image are no faster as one-slice CTAs
-// (3 x 301^2 x 257: 53 us against 50 us).
-bool bp_run_plain(const BpGeo &g, int geometry, int store, int nslices, int nangles, int turns)
-{
-    BpTune forced;
-    return nslices == 1 && store_bytes(store) == 4 && bp_runs_ok(g, geometry, nangles, turns) && !forced_tune(forced);
-}
-
 int bp_run_turns(const float *angles, int nangles)
 {
     int turns = 0;
@@ -672,8 +644,18 @@ int bp_run_turns(const float *angles, int nangles)
     return turns;
 }
 
+// The launch arguments from slice group group0 on (rows interleaved by slice).
+static BpArgs from_group(BpArgs a, int group0)
+{
+    a.filt += (size_t)group0 * a.nangles * a.Wg * 16;
+    a.img += (size_t)group0 * 4 * a.No * a.No;
+    if (a.den) a.den += (size_t)group0 * 4 * a.No * a.No;
+    a.nslices -= 4 * group0;
+    return a;
+}
+
 template <int GEOM, int STORE, bool UNIT, int G>
-static void launch_run_t(BpArgs a, int AB, int group0, int groups, cudaStream_t st)
+static void launch_run_t(const BpArgs &a, int AB, int groups, cudaStream_t st)
 {
     const size_t smem = kRunFixed + kRunStages * (size_t)AB * a.W * (G ? 16 * G : 4);
     RAFT_CHECK(smem <= kBpSmemMax && AB >= 1 && AB <= 32, "backprojector: staged window too large");
@@ -685,10 +667,6 @@ static void launch_run_t(BpArgs a, int AB, int group0, int groups, cudaStream_t 
         RAFT_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kBpSmemMax));
         configured = dev;
     }
-    a.filt += (size_t)group0 * a.nangles * a.Wg * 16;
-    a.img += (size_t)group0 * 4 * a.No * a.No;
-    if (a.den) a.den += (size_t)group0 * 4 * a.No * a.No;
-    a.nslices -= 4 * group0;
     dim3 grid((a.No + kRunTile - 1) / kRunTile, (a.No + kRunTile - 1) / kRunTile, groups / (G ? G : 1));
     ProfScope ps(PROF_BACKPROJECT, st);
     kern<<<grid, BP_THREADS, smem, st>>>(a, AB);
@@ -696,52 +674,36 @@ static void launch_run_t(BpArgs a, int AB, int group0, int groups, cudaStream_t 
 }
 
 template <int GEOM, int STORE, bool UNIT>
-static void launch_run_s(BpArgs a, const WindowLayout &win, cudaStream_t st)
+static void launch_run_s(BpArgs a, const WindowLayout &win, const BpSplit &sp, cudaStream_t st)
 {
-    if (!a.il) {   // one slice per CTA on plain rows
+    if (sp.one) {   // one slice on plain rows of four-byte elements
         if constexpr (STORE != STORE_PAIR_F32) {
             a.W = (win.Wrun + 3) & ~3;
-            launch_run_t<GEOM, STORE, UNIT, 0>(a, 32, 0, a.nslices, st);
+            launch_run_t<GEOM, STORE, UNIT, 0>(a, 32, 1, st);
         }
         return;
     }
-    // Sixteen or eight slices per thread share a position's arithmetic where that
-    // leaves every SM the two CTAs that fit it; else, and for what is left over,
-    // four.  32 x 2048^2 x 1800, nearest: 25.2, 26.2 and 31.5 ms per pass (the
-    // single-pixel kernel 31.5); linear interpolation, whose bins take twice the
-    // registers, gains nothing from sixteen (11.05 ms either way).
-    const int groups = (a.nslices + 3) / 4;
-    const long long tiles = (long long)((a.No + kRunTile - 1) / kRunTile) * ((a.No + kRunTile - 1) / kRunTile);
     a.W = win.Wrun;
-    int g0 = 0;
-    if constexpr (STORE == STORE_F32) {
-        const int n = groups / 4;
-        if (tiles * n >= 2 * 148) {
-            launch_run_t<GEOM, STORE, UNIT, 4>(a, 8, 0, 4 * n, st);
-            g0 = 4 * n;
-        }
-    }
-    if (const int n = (groups - g0) / 2; tiles * n >= 2 * 148) {
-        launch_run_t<GEOM, STORE, UNIT, 2>(a, 16, g0, 2 * n, st);
-        g0 += 2 * n;
-    }
-    if (g0 < groups) launch_run_t<GEOM, STORE, UNIT, 1>(a, 16, g0, groups - g0, st);
+    if constexpr (STORE == STORE_F32)
+        if (sp.g16) launch_run_t<GEOM, STORE, UNIT, 4>(a, 8, sp.g16, st);
+    if (sp.g8) launch_run_t<GEOM, STORE, UNIT, 2>(from_group(a, sp.g16), 16, sp.g8, st);
+    if (sp.g4) launch_run_t<GEOM, STORE, UNIT, 1>(from_group(a, sp.g16 + sp.g8), 16, sp.g4, st);
 }
 
-static void launch_run(BpArgs a, const WindowLayout &win, int geometry, int store, cudaStream_t st)
+static void launch_run(BpArgs a, const WindowLayout &win, const BpSplit &sp, int geometry, int store, cudaStream_t st)
 {
     const double umax = std::max(std::abs(win.wlo), std::abs(win.wlo + win.Wg));
     a.eps = 1e-3f + (geometry == GEOM_FBP_LIN ? 0.f : (float)(umax / (1 << 20)));
     switch (geometry) {
     case GEOM_FBP_REF:
         // bins of unit width (pixel size 1, the default): no multiplication by 1 / dt
-        if (a.dt == 1.f) launch_run_s<GEOM_FBP_REF, STORE_F32, true>(a, win, st);
-        else launch_run_s<GEOM_FBP_REF, STORE_F32, false>(a, win, st);
+        if (a.dt == 1.f) launch_run_s<GEOM_FBP_REF, STORE_F32, true>(a, win, sp, st);
+        else launch_run_s<GEOM_FBP_REF, STORE_F32, false>(a, win, sp, st);
         break;
-    case GEOM_EM_REF: launch_run_s<GEOM_EM_REF, STORE_F32, false>(a, win, st); break;
+    case GEOM_EM_REF: launch_run_s<GEOM_EM_REF, STORE_F32, false>(a, win, sp, st); break;
     default:
-        if (store == STORE_PAIR_BF16) launch_run_s<GEOM_FBP_LIN, STORE_PAIR_BF16, true>(a, win, st);
-        else launch_run_s<GEOM_FBP_LIN, STORE_PAIR_F32, true>(a, win, st);
+        if (store == STORE_PAIR_BF16) launch_run_s<GEOM_FBP_LIN, STORE_PAIR_BF16, true>(a, win, sp, st);
+        else launch_run_s<GEOM_FBP_LIN, STORE_PAIR_F32, true>(a, win, sp, st);
         break;
     }
 }
@@ -799,10 +761,160 @@ static bool forced_tune(BpTune &t)
     return false;
 }
 
-bool bp_forced_planar()
+// RAFT_BP_TUNE="run,K" forces the run kernel with K = 1, 4, 8 or 16 slices per thread
+// where the launch has such a form (tests); 0: not forced.
+static int forced_run()
+{
+    const char *e = std::getenv("RAFT_BP_TUNE");
+    int k = 0;
+    if (!e || std::sscanf(e, "run,%d", &k) != 1) return 0;
+    return k == 1 || k == 4 || k == 8 || k == 16 ? k : 0;
+}
+
+// ------------------------------------------------------------------------
+// which kernel takes which slices
+// ------------------------------------------------------------------------
+// What a launch costs, in us, measured on this kernel's own grid: an SM runs
+// `resident` blocks at a time; the last wave's k blocks per SM take fixed[k - 1] +
+// angle[k - 1] * (number of angles), each wave before it fixed[resident] + ....  Blocks
+// are 32 x 32 pixels (run kernel) or 64 x 32 (single-pixel kernel), times `slices`.
+// Fitted to the times of 400 - 2100 launches per row (96^2 - 2048^2 pixels, 48 - 1024
+// angles over [0, pi), 1 - 32 slices); the fit is off by 1 - 3 % (root mean square).
+struct BpCost {
+    int slices, width, resident;
+    float fixed[6], angle[6];
+    double time(int No, int nslices, int nangles) const
+    {
+        const long long blocks =
+            (long long)((No + width - 1) / width) * ((No + 31) / 32) * ((nslices + slices - 1) / slices);
+        const long long wave = 148LL * resident, before = (blocks - 1) / wave;
+        const int last = (int)((blocks - before * wave + 147) / 148);
+        auto t = [&](int k) { return fixed[k] + (double)angle[k] * nangles; };
+        return (double)before * t(resident) + t(last - 1);
+    }
+};
+// the single-pixel kernel untuned, and with one and four slices per block (FP32 pairs)
+enum { BP_SINGLE = 0, BP_SINGLE1, BP_SINGLE4, BP_ONE, BP_RUN4, BP_RUN8, BP_RUN16, BP_FORMS };
+// A few points behind the rows (us, single-pixel kernel | run kernel with 4, 8, 16
+// slices per thread), nearest sample, bins of unit width: 512^2 x 128 angles, 8 slices
+// 54 | 68, 54; x 720 257 | 267, 201; 1024^2 x 128, 16 slices 293 | 383, 322, 318;
+// x 720 1557 | 1661, 1326, 1301; one slice, 512^2 x 360: 105 | one-slice form 52.
+// No form is the best one everywhere: the run kernel's forms pay for turning their
+// accumulators and for the classes of slopes, and every grid pays for its last wave.
+static const BpCost kBpCost[4][BP_FORMS] = {
+    // nearest sample, bins of unit width
+    {{4, 64, 3, {-1.2f, -0.3f, 0.5f, 2.3f}, {0.267f, 0.347f, 0.465f, 0.448f}},
+     {},
+     {},
+     {1, 32, 4, {5.1f, 5.6f, 7.2f, 8.6f, 10.0f}, {0.071f, 0.101f, 0.141f, 0.185f, 0.164f}},
+     {4, 32, 3, {6.5f, 7.8f, 9.9f, 11.6f}, {0.115f, 0.174f, 0.25f, 0.223f}},
+     {8, 32, 2, {10.9f, 12.4f, 15.2f}, {0.155f, 0.255f, 0.232f}},
+     {16, 32, 2, {21.1f, 22.7f, 26.7f}, {0.3f, 0.499f, 0.449f}}},
+    // nearest sample, other bins (EM)
+    {{4, 64, 3, {-2.2f, -0.3f, 0.1f, 2.3f}, {0.247f, 0.333f, 0.458f, 0.443f}},
+     {},
+     {},
+     {1, 32, 4, {4.7f, 5.2f, 6.1f, 7.6f, 9.1f}, {0.073f, 0.106f, 0.152f, 0.199f, 0.177f}},
+     {4, 32, 3, {6.0f, 7.1f, 8.5f, 10.8f}, {0.12f, 0.185f, 0.27f, 0.24f}},
+     {8, 32, 2, {10.0f, 11.6f, 14.7f}, {0.157f, 0.258f, 0.233f}},
+     {16, 32, 2, {18.1f, 21.3f, 25.1f}, {0.302f, 0.494f, 0.448f}}},
+    // linear interpolation, BF16 pairs
+    {{4, 64, 3, {-2.0f, -0.9f, -0.7f, 1.7f}, {0.445f, 0.579f, 0.827f, 0.724f}},
+     {},
+     {},
+     {1, 32, 3, {5.7f, 6.1f, 7.0f, 9.5f}, {0.078f, 0.129f, 0.19f, 0.171f}},
+     {4, 32, 3, {7.2f, 8.2f, 9.5f, 10.9f}, {0.163f, 0.282f, 0.418f, 0.382f}},
+     {8, 32, 2, {12.9f, 14.4f, 15.6f}, {0.23f, 0.431f, 0.403f}},
+     {}},
+    // linear interpolation, FP32 (the single-pixel kernel: planar pairs; two slices per
+    // block, or what was tuned: one, two or four)
+    {{2, 64, 4, {-2.4f, -1.6f, -0.7f, -0.3f, 2.5f}, {0.404f, 0.462f, 0.587f, 0.751f, 0.654f}},
+     {1, 64, 5, {-2.4f, -1.9f, -1.1f, -1.0f, -1.0f, 2.2f}, {0.209f, 0.285f, 0.397f, 0.524f, 0.646f, 0.579f}},
+     {4, 64, 3, {-2.7f, -0.4f, 0.4f, 2.8f}, {0.685f, 0.791f, 0.993f, 0.93f}},
+     {},
+     {4, 32, 3, {7.6f, 8.1f, 9.9f, 11.2f}, {0.165f, 0.29f, 0.429f, 0.39f}},
+     {8, 32, 2, {12.8f, 14.2f, 15.0f}, {0.238f, 0.447f, 0.416f}},
+     {}},
+};
+constexpr double kNextLaunch = 5.0;   // a further launch of the same call (us)
+constexpr int kRunMinAngles = 48;     // below, the fit does not hold and nothing is gained
+
+// The run kernel's rule on positions needs pixels as wide as detector bins.  Turning
+// the accumulators costs about as much as three angles, so angle lists that change
+// the run axis more often than every 16 angles (scans in golden-ratio order) keep
+// the single-pixel kernel.
+static bool run_possible(const BpGeo &g, int geometry)
+{
+    if (geometry == GEOM_EM_REF) return g.dxy == g.dt;
+    return g.dx == g.dt && g.dy == g.dt && g.ratio == 1.0;
+}
+
+BpSplit bp_split(const BpGeo &g, int geometry, int store, int No, int nslices, int nangles, int turns)
+{
+    const int groups = (nslices + 3) / 4;
+    const bool f32 = geometry == GEOM_FBP_LIN && store == STORE_PAIR_F32, bf16 = geometry == GEOM_FBP_LIN && !f32;
+    const bool has16 = geometry != GEOM_FBP_LIN, has1 = !f32 && nslices == 1;
+    BpSplit best;
+    best.single = groups;
+    BpTune forced;
+    if (forced_tune(forced) || !run_possible(g, geometry) || nslices < 1) return best;
+    auto split = [&](bool use16, bool use8, bool use4) {
+        BpSplit s;
+        if (use16) s.g16 = groups / 4 * 4;
+        if (use8) s.g8 = (groups - s.g16) / 2 * 2;
+        const int rest = groups - s.g16 - s.g8;
+        (use4 ? s.g4 : s.single) = rest;
+        return s;
+    };
+    if (const int k = forced_run(); k) {
+        if (k != 1) return split(k == 16 && has16, k >= 8, true);
+        if (!has1) return best;
+        best = BpSplit();
+        best.one = true;
+        return best;
+    }
+    if (nangles < kRunMinAngles || turns > nangles / 16 + 2) return best;
+    const BpCost *cost = kBpCost[f32 ? 3 : bf16 ? 2 : (geometry == GEOM_EM_REF || g.dt != 1.f) ? 1 : 0];
+    auto form_time = [&](int form, int slices) { return cost[form].time(No, slices, nangles); };
+    double t_best = form_time(BP_SINGLE, nslices);
+    if (f32 && nslices >= 8)   // tuned
+        t_best = std::min({t_best, form_time(BP_SINGLE1, nslices), form_time(BP_SINGLE4, nslices)});
+    if (has1)
+        if (const double t = form_time(BP_ONE, 1); t < t_best) {
+            t_best = t;
+            best = BpSplit();
+            best.one = true;
+        }
+    for (int m = 0; m < 8; m++) {
+        const BpSplit s = split(m & 1, m & 2, m & 4);
+        if (s.single == groups || ((m & 1) && !has16)) continue;
+        if (f32 && s.single) continue;   // interleaved single floats are the run kernel's alone
+        double t = -kNextLaunch;
+        int left = nslices;
+        auto add = [&](int form, int n) {
+            if (!n) return;
+            t += kNextLaunch + form_time(form, std::min(left, 4 * n));
+            left -= 4 * n;
+        };
+        add(BP_RUN16, s.g16);
+        add(BP_RUN8, s.g8);
+        add(BP_RUN4, s.g4);
+        add(BP_SINGLE, s.single);
+        if (t < t_best) {
+            t_best = t;
+            best = s;
+        }
+    }
+    return best;
+}
+
+// Interleaved by slice: what the run kernel reads (but for a single slice), and the
+// single-pixel kernel's four-byte elements.
+bool bp_interleaved(const BpSplit &s, int store)
 {
     BpTune t;
-    return forced_tune(t) && t.S != 4;
+    if (s.one || (forced_tune(t) && t.S != 4)) return false;
+    return s.g16 || s.g8 || s.g4 || store_bytes(store) == 4;
 }
 
 // Pick (S, AB) for this configuration: the cached choice, else time every
@@ -932,26 +1044,20 @@ size_t bp_il_bytes(int nslices, int nangles, int Wg, int esize)
 void launch_backproject(const BpLaunch &bl, cudaStream_t st)
 {
     if (bl.nslices <= 0 || bl.nangles <= 0) return;
-    const BpArgs a = to_args(bl);
+    BpArgs a = to_args(bl);
     const int store = bl.geometry == GEOM_FBP_LIN ? bl.store : STORE_F32;
-    if (bl.il_ready) {
-        // rows interleaved by slice in groups of four
-        BpArgs a_il = a;
-        a_il.filt = reinterpret_cast<const unsigned char *>(bl.il_ws);
-        a_il.il = 1;
-        if (bp_runs_ok(bl.geo, bl.geometry, bl.nangles, bl.turns)) {
-            launch_run(a_il, bl.win, bl.geometry, store, st);
-            return;
-        }
+    if (!bl.il_ready && !bl.split.one) {   // planar rows
+        launch_bp_any(a, bl.geometry, store, choose_tune(a, bl.geometry, store, st), st);
+        return;
+    }
+    a.il = bl.il_ready;
+    if (!bl.split.single || bl.split.g16 || bl.split.g8 || bl.split.g4)
+        launch_run(a, bl.win, bl.split, bl.geometry, store, st);
+    if (bl.split.single) {
         RAFT_CHECK(a.esize == 4, "backprojector: interleaved rows need 4-byte elements");
-        launch_bp_any(a_il, bl.geometry, store, choose_tune(a_il, bl.geometry, store, st, true), st);
-        return;
+        const BpArgs r = from_group(a, bl.split.g16 + bl.split.g8 + bl.split.g4);
+        launch_bp_any(r, bl.geometry, store, choose_tune(r, bl.geometry, store, st, true), st);
     }
-    if (bp_run_plain(bl.geo, bl.geometry, store, bl.nslices, bl.nangles, bl.turns)) {
-        launch_run(a, bl.win, bl.geometry, store, st);
-        return;
-    }
-    launch_bp_any(a, bl.geometry, store, choose_tune(a, bl.geometry, store, st), st);
 }
 
 // ------------------------------------------------------------------------

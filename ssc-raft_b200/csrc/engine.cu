@@ -338,24 +338,22 @@ size_t fbp_rows_bytes(const FbpPrepared &fp, int nslices)
     return (size_t)nslices * fp.cfg.nangles * fp.win.Wg * store_bytes(fp.cfg.store);
 }
 
-bool fbp_fused_il(const FbpPrepared &fp)
+size_t fbp_ws_bytes(const FbpPrepared &fp, int nslices)
 {
-    return fbp_il_bytes(fp, 1) > 0 && !bp_forced_planar();
+    return std::max(fbp_rows_bytes(fp, nslices), bp_il_bytes(nslices, fp.cfg.nangles, fp.win.Wg, 4));
 }
 
-void fbp_chunk(DeviceState &ds, const FbpPrepared &fp, const FbpTables &tb, const float *d_sino, float *d_img,
-               int nslices, void *d_rows, cudaStream_t st, void *d_il)
+void fbp_chunk(const FbpPrepared &fp, const FbpTables &tb, const float *d_sino, float *d_img, int nslices,
+               void *d_rows, cudaStream_t st, bool il)
 {
-    (void)ds;
     if (nslices <= 0) return;
-    // with the interleave workspace and 4-byte elements the filter writes the
-    // four-slice interleaved rows the backprojector stages, directly
-    const bool plain = d_il && bp_run_plain(fp.geo, fp.cfg.geometry, fp.cfg.store, nslices, fp.cfg.nangles, fp.turns);
-    const bool fused = d_il && !plain && fbp_fused_il(fp);
-    if (plain) d_rows = d_il;   // plain rows in the interleaved ones' place
+    BpSplit split;
+    if (il) split = bp_split(fp.geo, fp.cfg.geometry, fp.cfg.store, fp.No, nslices, fp.cfg.nangles, fp.turns);
+    // the filter writes the four-slice interleaved rows the backprojector stages, directly
+    const bool fused = il && bp_interleaved(split, fp.cfg.store);
     FilterLaunch fl;
     fl.sino = d_sino;
-    fl.out = fused ? d_il : d_rows;
+    fl.out = d_rows;
     fl.interleaved = fused ? 1 : 0;
     fl.wt = tb.wt;
     fl.nrows = nslices * fp.cfg.nangles;
@@ -367,7 +365,7 @@ void fbp_chunk(DeviceState &ds, const FbpPrepared &fp, const FbpTables &tb, cons
     fl.store = fused && fp.cfg.store == STORE_PAIR_F32 ? (int)STORE_F32 : fp.cfg.store;
     launch_filter(*fp.plan, fl, st);
     BpLaunch bl;
-    bl.filt = fused ? nullptr : d_rows;
+    bl.filt = d_rows;
     bl.img = d_img;
     bl.No = fp.No;
     bl.nangles = fp.cfg.nangles;
@@ -381,17 +379,9 @@ void fbp_chunk(DeviceState &ds, const FbpPrepared &fp, const FbpTables &tb, cons
     bl.csd = tb.csd;
     bl.snd = tb.snd;
     bl.err = tb.err;
-    bl.il_ws = d_il;
     bl.il_ready = fused ? 1 : 0;
-    bl.turns = fp.turns;
+    bl.split = split;
     launch_backproject(bl, st);
-}
-
-size_t fbp_il_bytes(const FbpPrepared &fp, int nslices)
-{
-    // pairs of floats are read by the run kernel only (from single floats)
-    const bool il = store_bytes(fp.cfg.store) == 4 || bp_runs_ok(fp.geo, fp.cfg.geometry, fp.cfg.nangles, fp.turns);
-    return il ? bp_il_bytes(nslices, fp.cfg.nangles, fp.win.Wg, 4) : 0;
 }
 
 static void check_device_flag(const int *d_err, const char *what)
@@ -414,10 +404,9 @@ void fbp_host_slab(const FbpConfig &cfg, int device, float *obj, const float *to
     const size_t in_ps = (size_t)cfg.nangles * cfg.nrays * sizeof(float);
     const size_t out_ps = (size_t)fp.No * fp.No * sizeof(float);
     const int chunk = auto_chunk(nslices, in_ps, cfg.blocksize);
-    void *il = fbp_il_bytes(fp, chunk) ? ds.il.get(fbp_il_bytes(fp, chunk)) : nullptr;
-    void *rows = (il && fbp_fused_il(fp)) ? nullptr : ds.rows.get(fbp_rows_bytes(fp, chunk));
+    void *rows = ds.il.get(fbp_ws_bytes(fp, chunk));
     run_pipeline(ds, nslices, chunk, in_ps, out_ps, tomo, obj, [&](void *din, void *dout, int ns, cudaStream_t st) {
-        fbp_chunk(ds, fp, tb, (const float *)din, (float *)dout, ns, rows, st, il);
+        fbp_chunk(fp, tb, (const float *)din, (float *)dout, ns, rows, st, true);
     });
     check_device_flag(tb.err, "FBP");
 }
@@ -706,15 +695,10 @@ void em_chunk(DeviceState &ds, const EmPrepared &ep, int kind, const float *d_da
     bl.cs = cs;
     bl.sn = sn;
     bl.err = err;
-    bl.turns = bp_run_turns(h_angles, A);
-    // one slice: plain rows
-    const bool plain = bp_run_plain(ep.geo, GEOM_EM_REF, STORE_F32, nslices, A, bl.turns);
-    if (plain) {
-        bl.filt = rows;
-    } else {
-        bl.il_ws = rows;
-        bl.il_ready = 1;
-    }
+    bl.filt = rows;
+    bl.split = bp_split(ep.geo, GEOM_EM_REF, STORE_F32, N, nslices, A, bp_run_turns(h_angles, A));
+    const bool plain = bl.split.one;   // one slice: plain rows
+    bl.il_ready = plain ? 0 : 1;
 
     // sensitivity image: BP of the counts (tEM, em_rt.cu:178) or of ones (eEM, :343)
     const float *counts = kind == 0 ? d_data : nullptr;

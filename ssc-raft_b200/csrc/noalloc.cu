@@ -200,12 +200,11 @@ extern "C" int raft_fbp_device_noalloc(int gpu, float *d_obj, const float *d_tom
         }
 
         // filter + backprojection, `chunk` slices at a time through the rows region
-        DeviceState unused;
         void *rows = base + o_rows;
         const size_t tomo_ps = (size_t)A * N, obj_ps = (size_t)No * No;
         for (int s0 = 0; s0 < cfg.nslices; s0 += chunk) {
             const int ns = std::min(chunk, cfg.nslices - s0);
-            fbp_chunk(unused, fp, tb, d_tomogram + tomo_ps * s0, d_obj + obj_ps * s0, ns, rows, st);
+            fbp_chunk(fp, tb, d_tomogram + tomo_ps * s0, d_obj + obj_ps * s0, ns, rows, st, false);
         }
         int flag = 0;
         RAFT_CUDA(cudaMemcpyAsync(&flag, tb.err, sizeof(int), cudaMemcpyDeviceToHost, st));

@@ -150,6 +150,14 @@ struct BpPlanInput {
 
 WindowLayout plan_window(const BpPlanInput &in);
 
+// How a launch's slices are shared out, in groups of four in this order: by sixteen,
+// eight and four slices per thread of the run kernel, then the single-pixel kernel.
+struct BpSplit {
+    int g16 = 0, g8 = 0, g4 = 0;   // groups
+    int single = 0;                // groups
+    bool one = false;              // one slice on plain rows by the run kernel
+};
+
 struct BpLaunch {
     const void *filt = nullptr;   // window rows [nslices*nangles][Wg]
     float *img = nullptr;         // [nslices][No][No]
@@ -161,26 +169,18 @@ struct BpLaunch {
     const float *cs = nullptr, *sn = nullptr;     // FP32 angle tables
     const double *csd = nullptr, *snd = nullptr;  // FP64 angle tables
     int *err = nullptr;                           // device error flag
-    // 1: il_ws holds the rows interleaved by slice in groups of four
-    //    (bp_il_bytes; filt unused)
+    // 1: filt holds the rows interleaved by slice in groups of four (bp_il_bytes)
     int il_ready = 0;
-    const void *il_ws = nullptr;
-    // changes of the run axis along the angle list (bp_run_turns)
-    int turns = 1 << 30;
+    BpSplit split;                                // of interleaved rows, or one slice's plain ones
 };
 
 void launch_backproject(const BpLaunch &bl, cudaStream_t st);
 size_t bp_il_bytes(int nslices, int nangles, int Wg, int esize);
-// Times the run axis changes between neighbouring angles, and whether
-// interleaved rows go through the run kernel (which takes linear
-// interpolation's FP32 rows as single floats).
+// Times the run axis changes between neighbouring angles.
 int bp_run_turns(const float *angles, int nangles);
-bool bp_runs_ok(const BpGeo &g, int geometry, int nangles, int turns);
-// Whether a launch of nslices slices takes plain rows to the run kernel.
-bool bp_run_plain(const BpGeo &g, int geometry, int store, int nslices, int nangles, int turns);
-// True when RAFT_BP_TUNE forces a shape of fewer than four slices per CTA
-// (which reads plain, not interleaved, rows).
-bool bp_forced_planar();
+// The split of nslices slices, and whether the rows are interleaved for it.
+BpSplit bp_split(const BpGeo &g, int geometry, int store, int No, int nslices, int nangles, int turns);
+bool bp_interleaved(const BpSplit &s, int store);
 
 // Backprojector launch shape chosen by the autotuner: S slices per CTA
 // (sharing each pixel's position arithmetic) and AB angles per pipeline stage.

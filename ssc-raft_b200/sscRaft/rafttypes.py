@@ -98,6 +98,8 @@ libraft.raft_slab_partition.argtypes = [_I, _I, _P, _P]
 libraft.raft_slab_partition.restype = _I
 libraft.raft_plan_window.argtypes = [_P, _P, _I, _I, _P]
 libraft.raft_plan_window.restype = _I
+libraft.raft_bp_split.argtypes = [_P, _P, _P, _I, _I, _I, _P]
+libraft.raft_bp_split.restype = _I
 libraft.raft_fast_sincos.argtypes = [_I, _P, _I, _I, _P, _P]
 libraft.raft_fast_sincos.restype = _I
 

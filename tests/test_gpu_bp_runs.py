@@ -1,14 +1,16 @@
 """The backprojector's run kernel (pixels in runs along the image axis on which
-the detector coordinate moves slowest; one, four, eight or sixteen slices per CTA) against
+the detector coordinate moves slowest; one, four, eight or sixteen slices per thread) against
 the single-pixel kernel: both compute every pixel's bin with the same
 single-precision expressions and add the angles in the same order, so images are
-equal bit for bit.  RAFT_BP_TUNE="2,16" selects the single-pixel kernel on plain
-rows.  The list has sizes around the 32-pixel tile, angle counts around the 16-
-and 32-angle stages, slices that leave one, two and three groups of four (sixteen
-or eight slices per CTA need 296 CTAs: 704^2 and 1100^2), bins narrower and wider than 1,
-detectors without padding (negative bins at the corners), scans over 2 pi,
-backwards and with the slopes where the slope classes meet, and a scan that
-changes the run axis too often for the run kernel."""
+equal bit for bit.  RAFT_BP_TUNE="2,16" selects the single-pixel kernel on plain rows,
+"4,16" on interleaved ones, "run,K" the run kernel with K slices per thread;
+raft_bp_split says which kernel a call takes, and is asked before each comparison.  The
+list has sizes around the 32-pixel tile, angle counts around the 16- and 32-angle
+stages, slices that leave one, two and three groups of four behind the wider forms,
+bins narrower and wider than 1, detectors without padding (negative bins at the
+corners), scans over 2 pi, backwards and with the slopes where the slope classes
+meet, and a scan that changes the run axis too often for the rule to take the run
+kernel."""
 import ctypes
 import os
 
@@ -53,11 +55,33 @@ def _fbp(sino, ang, N, pad, pixel, offset, ftype, geometry, store):
     return out
 
 
+def _split(N, ang, n, pixel, geometry, store):
+    """(groups by 16, by 8, by 4, single-pixel groups, one slice on plain rows)"""
+    from sscRaft.rafttypes import _ptr, libraft
+    pf = np.array([0, 0, 1, 0, pixel, pixel, 0], np.float32)
+    pi = np.array([N, len(ang), n, N, 0, 0, 0, 1 if geometry == 2 else 5, 1 if geometry == 2 else 0, 0], np.int32)
+    out = np.zeros(5, np.int32)
+    assert libraft.raft_bp_split(_ptr(pf), _ptr(pi), _ptr(ang), geometry, store, n, _ptr(out)) == 0
+    return tuple(int(v) for v in out)
+
+
+def _forms(n, geometry, store):
+    """Slices per thread that n slices can take, and the split each must give."""
+    g = -(-n // 4)
+    forms = {4: (0, 0, g, 0, 0), 8: (0, g // 2 * 2, g % 2, 0, 0)}
+    if geometry != 1:
+        forms[16] = (g // 4 * 4, g % 4 // 2 * 2, g % 2, 0, 0)
+    if n == 1 and (geometry, store) != (1, 1):
+        forms[1] = (0, 0, 0, 0, 1)
+    return {k: v for k, v in forms.items() if k <= 4 or v[0] or v[1]}
+
+
 @pytest.mark.parametrize("N,A,n,pad,offset,pixel,kind", [
     (31, 15, 1, 2, 0.5, 1.0, "pi"), (32, 16, 2, 1, 0.0, 1.0, "pi"), (33, 17, 5, 0, 0.3, 1.0, "pi"),
     (64, 32, 4, 2, 0.0, 0.5, "2pi"), (97, 33, 1, 0, 0.0, 2.0, "back"), (129, 100, 9, 0, -1.5, 1.0, "edges"),
     (257, 100, 1, 1, 1.25, 0.7, "edges"), (300, 61, 6, 2, 1.25, 1.0, "back"), (704, 48, 8, 2, 3.5, 1.0, "pi"),
-    (1100, 40, 13, 1, -2.0, 1.0, "2pi"), (601, 37, 29, 0, 0.0, 1.0, "pi"), (100, 64, 4, 2, 0.0, 1.0, "golden")])
+    (1100, 40, 13, 1, -2.0, 1.0, "2pi"), (601, 37, 29, 0, 0.0, 1.0, "pi"), (129, 143, 17, 0, 0.0, 1.0, "edges"),
+    (257, 161, 30, 1, 0.5, 0.7, "2pi")])
 def test_runs_equal_single_pixels(restore_env, N, A, n, pad, offset, pixel, kind):
     import torch
     ang = _angles(kind, A)
@@ -65,9 +89,31 @@ def test_runs_equal_single_pixels(restore_env, N, A, n, pad, offset, pixel, kind
     sino = torch.randn((n, len(ang), N), generator=g, device="cuda")
     for geometry, store in ((0, 0), (1, 1), (1, 2)):
         os.environ["RAFT_BP_TUNE"] = "2,16"
+        assert _split(N, ang, n, pixel, geometry, store) == (0, 0, 0, -(-n // 4), 0)
         ref = _fbp(sino, ang, N, pad, pixel, offset, 5, geometry, store)
+        for k, split in _forms(n, geometry, store).items():
+            os.environ["RAFT_BP_TUNE"] = "run,%d" % k
+            assert _split(N, ang, n, pixel, geometry, store) == split
+            assert torch.equal(_fbp(sino, ang, N, pad, pixel, offset, 5, geometry, store), ref), (geometry, store, k)
         del os.environ["RAFT_BP_TUNE"]
         assert torch.equal(_fbp(sino, ang, N, pad, pixel, offset, 5, geometry, store), ref), (geometry, store)
+
+
+@pytest.mark.parametrize("N,A,n,kind,want", [
+    (512, 360, 1, "pi", "one"), (300, 128, 4, "pi", "g4"), (512, 256, 16, "pi", "g16"), (512, 256, 28, "pi", "mixed"),
+    (512, 720, 12, "pi", "mixed"), (300, 47, 4, "pi", "single"), (300, 300, 4, "golden", "single")])
+def test_the_rules_choice_equals_single_pixels(restore_env, N, A, n, kind, want):
+    """Without forcing, one call of every kind that the rule makes (nearest sample)."""
+    import torch
+    ang = _angles(kind, A)
+    got = _split(N, ang, n, 1.0, 0, 0)
+    assert {"one": got[4], "g4": got[2], "g16": got[0], "mixed": got[0] + got[1] > 0 and got[2] + got[3] > 0,
+            "single": got == (0, 0, 0, -(-n // 4), 0)}[want], got
+    g = torch.Generator(device="cuda").manual_seed(N + n)
+    sino = torch.randn((n, len(ang), N), generator=g, device="cuda")
+    out = _fbp(sino, ang, N, 1, 1.0, 0.25, 5, 0, 0)
+    os.environ["RAFT_BP_TUNE"] = "2,16"
+    assert torch.equal(_fbp(sino, ang, N, 1, 1.0, 0.25, 5, 0, 0), out)
 
 
 @pytest.mark.parametrize("n", [1, 4, 8, 16])
@@ -82,10 +128,46 @@ def test_non_finite_bins_stay_where_they_are(restore_env, n):
     sino[:, 9, 640] = float("nan")
     os.environ["RAFT_BP_TUNE"] = "2,16"
     ref = _fbp(sino, ang, N, 1, 1.0, 0.0, 0, 0, 0)
-    del os.environ["RAFT_BP_TUNE"]
-    out = _fbp(sino, ang, N, 1, 1.0, 0.0, 0, 0, 0)
     assert not torch.isfinite(ref).all() and torch.isfinite(ref).float().mean() > 0.9
-    assert torch.equal(torch.nan_to_num(out, 123.0, 456.0, -456.0), torch.nan_to_num(ref, 123.0, 456.0, -456.0))
+    for k, split in _forms(n, 0, 0).items():
+        os.environ["RAFT_BP_TUNE"] = "run,%d" % k
+        assert _split(N, ang, n, 1.0, 0, 0) == split
+        out = _fbp(sino, ang, N, 1, 1.0, 0.0, 0, 0, 0)
+        assert torch.equal(torch.nan_to_num(out, 123.0, 456.0, -456.0), torch.nan_to_num(ref, 123.0, 456.0, -456.0)), k
+
+
+def _em(kind, data, flat, ang, N, iters):
+    import torch
+    from sscRaft.rafttypes import _ptr, libraft
+    obj = torch.ones((data.shape[0], N, N), device="cuda")
+    assert libraft.raft_em_device(kind, 0, _p(obj), _p(data), _p(flat) if kind == 0 else None, _ptr(ang), N, len(ang),
+                                  data.shape[0], iters, None, 1, None) == 0
+    return obj
+
+
+@pytest.mark.parametrize("N,A,n,kind", [(97, 33, 1, 0), (161, 100, 6, 1), (300, 143, 18, 0), (129, 64, 29, 1)])
+def test_em_runs_equal_single_pixels(restore_env, N, A, n, kind):
+    """EM with every form of the run kernel, with the rule's choice and on an angle
+    list in golden-ratio order, against the single-pixel kernel."""
+    import torch
+    g = torch.Generator(device="cuda").manual_seed(N)
+    data = (0.2 + 0.8 * torch.rand((n, A, N), generator=g, device="cuda")).contiguous()
+    flat = torch.ones((n, N), device="cuda")
+
+    def same(a, b):          # steps between angles out of order are negative weights: EM overflows there
+        return torch.equal(torch.isnan(a), torch.isnan(b)) and torch.equal(torch.nan_to_num(a), torch.nan_to_num(b))
+
+    for order in ("pi", "golden"):
+        ang = _angles(order, A)
+        os.environ["RAFT_BP_TUNE"] = "4,16"
+        assert _split(N, ang, n, 1.0, 2, 0) == (0, 0, 0, -(-n // 4), 0)
+        ref = _em(kind, data, flat, ang, N, 2)
+        for k, split in _forms(n, 2, 0).items():
+            os.environ["RAFT_BP_TUNE"] = "run,%d" % k
+            assert _split(N, ang, n, 1.0, 2, 0) == split
+            assert same(_em(kind, data, flat, ang, N, 2), ref), (order, k)
+        del os.environ["RAFT_BP_TUNE"]
+        assert same(_em(kind, data, flat, ang, N, 2), ref), order
 
 
 @pytest.mark.parametrize("kind", [0, 1])

@@ -1,7 +1,9 @@
 """Every backprojector launch shape the autotuner may pick (S slices per CTA,
 AB angles per pipeline stage) gives bit-identical images: the per-pixel
 accumulation order over angles does not depend on the shape.  The shape is
-forced with RAFT_BP_TUNE="S,AB"."""
+forced with RAFT_BP_TUNE="S,AB", which selects the single-pixel kernel; without it (None)
+the rule's choice runs.  EM keeps its rows interleaved by slice, so its single-pixel
+kernel has the two S = 4 shapes only; the other entries run its default one."""
 import ctypes
 import os
 
@@ -41,13 +43,15 @@ def test_fbp_shapes_bit_identical(restore_env):
     pi = np.array([N, A, n, N, 2, 0, 0, 5, 0, 0], np.int32)
     for geometry, store in ((0, 0), (1, 1), (1, 2)):
         outs = {}
-        for c in CANDIDATES:
-            os.environ["RAFT_BP_TUNE"] = c
+        for c in CANDIDATES + [None]:
+            os.environ.pop("RAFT_BP_TUNE", None)
+            if c:
+                os.environ["RAFT_BP_TUNE"] = c
             out = torch.empty((n, N, N), device="cuda")
             assert libraft.raft_fbp_device(0, _p(out), _p(sino), _ptr(ang), _ptr(pf), _ptr(pi), geometry, store,
                                            None) == 0
             outs[c] = out
-        for c in CANDIDATES[1:]:
+        for c in CANDIDATES[1:] + [None]:
             assert torch.equal(outs[c], outs[CANDIDATES[0]]), (geometry, store, c)
 
 
@@ -64,11 +68,13 @@ def test_em_shapes_bit_identical(restore_env):
     trans = torch.exp(-proj * (3.0 / proj.amax())).contiguous()
     flat = torch.ones((n, N), device="cuda")
     outs = {}
-    for c in CANDIDATES:
-        os.environ["RAFT_BP_TUNE"] = c
+    for c in CANDIDATES + [None]:
+        os.environ.pop("RAFT_BP_TUNE", None)
+        if c:
+            os.environ["RAFT_BP_TUNE"] = c
         obj = torch.ones((n, N, N), device="cuda")
         assert libraft.raft_em_device(0, 0, _p(obj), _p(trans), _p(flat), _ptr(ang), N, A, n, iters, None, 1,
                                       None) == 0
         outs[c] = obj
-    for c in CANDIDATES[1:]:
+    for c in CANDIDATES[1:] + [None]:
         assert torch.equal(outs[c], outs[CANDIDATES[0]]), c
