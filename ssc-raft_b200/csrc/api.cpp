@@ -688,7 +688,7 @@ int raft_radon_device(int gpu, float *d_out, const float *d_phantom, const float
         cudaStream_t st = resolve_stream(ds, stream, ds.s_comp);
         float *d_ang = (float *)ds.angles.get(sizeof(float) * nangles);
         RAFT_CUDA(cudaMemcpyAsync(d_ang, angles, sizeof(float) * nangles, cudaMemcpyHostToDevice, st));
-        void *scratch = ds.imgT.get(proj_scratch_bytes(nx, ny, nslices));
+        void *scratch = ds.imgT.get(proj_scratch_bytes(nx, ny, nslices, nangles));
         ProjLaunch pl;
         pl.img = d_phantom;
         pl.out = d_out;

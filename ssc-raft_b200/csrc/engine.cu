@@ -621,7 +621,7 @@ void radon_host_slab(int device, float *proj, const float *img, const float *ang
     const size_t in_ps = (size_t)nx * ny * sizeof(float);
     const size_t out_ps = (size_t)nangles * nrays * sizeof(float);
     const int chunk = auto_chunk(nslices, std::max(in_ps, out_ps), 0);
-    void *scratch = ds.imgT.get(proj_scratch_bytes(nx, ny, chunk));
+    void *scratch = ds.imgT.get(proj_scratch_bytes(nx, ny, chunk, nangles));
     run_pipeline(ds, nslices, chunk, in_ps, out_ps, img, proj, [&](void *din, void *dout, int ns, cudaStream_t st) {
         ProjLaunch pl;
         pl.img = (const float *)din;
@@ -708,7 +708,7 @@ void em_chunk(DeviceState &ds, const EmPrepared &ep, int kind, const float *d_da
     bl.den = nullptr;
     launch_backproject(bl, st);
 
-    void *scratch = ds.imgT.get(proj_scratch_bytes(N, N, nslices));
+    void *scratch = ds.imgT.get(proj_scratch_bytes(N, N, nslices, A));
     ProjLaunch pl;
     pl.img = d_obj;
     pl.out = rows;

@@ -25,6 +25,7 @@
 #include "ptx.hpp"
 #include "profile.hpp"
 
+#include <algorithm>
 #include <cstdlib>
 #include <type_traits>
 
@@ -74,6 +75,11 @@ __device__ __forceinline__ void ldg_v8(const float *p, float (&w)[8])
                  : "l"(p));
 }
 
+// Rows of the interleaved copies start on 128-byte lines.  Rows of 32-byte pixels that
+// do not cost every warp load more lines: 8 x 901^2 x 360 621 us with rows nx pixels
+// apart, 485 now.
+__host__ __device__ __forceinline__ int il_pitch(int n) { return (n + 3) & ~3; }
+
 template <int EM, int EPI, int S, int IL, int RW, int PH, int BRS>
 __device__ __forceinline__ void project_block(const ProjLaunch &p, const int bx, const int by, const int bz)
 {
@@ -97,10 +103,12 @@ __device__ __forceinline__ void project_block(const ProjLaunch &p, const int bx,
         const float ctheta = __cosf(ang);
         const float stheta = __sinf(ang);
         const bool steep = (IL ? p.ilT : p.imgT) && fabsf(stheta) > fabsf(ctheta);
-        const float *img = IL ? (steep ? p.ilT : p.il) + (size_t)bz * plane * 8
+        // address = Y*nx + X (row-major) or X*ny + Y (transposed), rows of interleaved
+        // copies il_pitch apart
+        const int px = IL ? il_pitch(nx) : nx, py = IL ? il_pitch(ny) : ny;
+        const float *img = IL ? (steep ? p.ilT + (size_t)bz * nx * py * 8 : p.il + (size_t)bz * ny * px * 8)
                               : (steep ? p.imgT : p.img) + (size_t)k0 * plane;
-        // address = Y*nx + X (row-major) or X*ny + Y (transposed)
-        const int sy = steep ? 1 : nx, sx = steep ? ny : 1;
+        const int sy = steep ? 1 : px, sx = steep ? py : 1;
         // This lane's samples (m = ph, ph + PH, ...) are processed four at a
         // time: the four positions and pixel loads are issued together
         // (independent, so their latency overlaps), then added in sample order.
@@ -110,7 +118,8 @@ __device__ __forceinline__ void project_block(const ProjLaunch &p, const int bx,
             if constexpr (IL) {
                 // two samples' positions and two slices' sums per instruction (the
                 // lanes round as the scalar instructions do); the sample number is
-                // counted in float, exactly.  24 x 1024^2 x 900: 4400 -> 4323 us.
+                // counted in float, exactly.  24 x 1024^2 x 900: 4400 -> 4104 us (with rows on
+                // 128-byte lines and four blocks per SM).
                 const u64 d2 = pack2(d0, d0), na2 = pack2(-ay0, -ay0), t2 = pack2(t, t), c2 = pack2(ctheta, ctheta);
                 const u64 s2 = pack2(stheta, stheta), ns2 = pack2(-stheta, -stheta), one2 = pack2(1.f, 1.f);
                 const float rx = __fdividef(1.0f, ddx), ry = __fdividef(1.0f, ddy);   // a / ddx is a times this
@@ -119,7 +128,7 @@ __device__ __forceinline__ void project_block(const ProjLaunch &p, const int bx,
 #pragma unroll
                 for (int q = 0; q < 4; q++) sum[q] = 0ull;
                 u64 m2 = pack2((float)ph, (float)(ph + PH));   // the next two sample numbers
-                constexpr int U = 4;   // samples in flight (6, 8 and 12 measured slower: 4350 - 4480 us)
+                constexpr int U = 4;   // samples in flight (6, 8 and 12 measured slower)
                 auto sample2 = [&](u64 mm, float (&w0)[8], float (&w1)[8]) {
                     const u64 s = fma2(mm, d2, na2);
                     const u64 x = mul2(add2(fma2(t2, c2, mul2(s, ns2)), one2), rx2);
@@ -318,7 +327,11 @@ __device__ __forceinline__ void project_block(const ProjLaunch &p, const int bx,
 }
 
 template <int EM, int EPI, int S, int IL, int RW, int PH, int BRS>
-__global__ void __launch_bounds__(32 * PJ_WARPS)
+// Four blocks per SM on interleaved images (24 x 1024^2 x 900: 4104 us; three blocks:
+// 4169, and launches of few blocks, 800^2 x 45, up to a quarter slower for their second
+// wave; 53 registers, the compiler's choice for EM: 16 x 1024^2 x 900 tEM 15.18 ->
+// 15.69 ms); the compiler's choice on planar ones (a bound of one block costs 7 - 17 %).
+__global__ void __launch_bounds__(32 * PJ_WARPS, IL ? 4 : 0)
 project_kernel(const ProjLaunch p)
 {
     project_block<EM, EPI, S, IL, RW, PH, BRS>(p, blockIdx.x, blockIdx.y, blockIdx.z);
@@ -441,7 +454,7 @@ void launch_transpose(const float *in, float *out, int nx, int ny, int nslices, 
 }
 
 // Slice-interleaved copies of groups of 8 planes, row-major and transposed:
-// il[g][y][x][s] = ilT[g][x][y][s] = in[8g + s][y][x] (zero where 8g + s is
+// il[g][y][x][s] = ilT[g][x][y][s] = in[8g + s][y][x] (rows il_pitch apart; zero where 8g + s is
 // past the last plane), plus the eight zeros that samples outside the image
 // read.  One 32 x TY pixel tile of all 8 planes per block: TY = 32, or 8 where
 // that would leave SMs without a block (301^2: 100 blocks, 10.9 us).
@@ -464,8 +477,9 @@ interleave_kernel(const float *__restrict__ in, float *__restrict__ il, float *_
         }
     }
     __syncthreads();
-    float *o = il + (size_t)g * plane * 8;
-    float *oT = ilT + (size_t)g * plane * 8;
+    const int px = il_pitch(nx), py = il_pitch(ny);
+    float *o = il + (size_t)g * ny * px * 8;
+    float *oT = ilT + (size_t)g * nx * py * 8;
     auto put = [&](float *p, int r, int c) {
         float4 *d = reinterpret_cast<float4 *>(p);
         d[0] = make_float4(tile[0][r][c], tile[1][r][c], tile[2][r][c], tile[3][r][c]);
@@ -473,42 +487,63 @@ interleave_kernel(const float *__restrict__ in, float *__restrict__ il, float *_
     };
     for (int r = threadIdx.y; r < TY; r += 8) {
         const int y = by + r, x = bx + tx;
-        if (x < nx && y < ny) put(o + ((size_t)y * nx + x) * 8, r, tx);
+        if (x < nx && y < ny) put(o + ((size_t)y * px + x) * 8, r, tx);
     }
     // transposed: TY consecutive y per x
     for (int e = threadIdx.y * 32 + tx; e < 32 * TY; e += 256) {
         const int c = e / TY, r = e % TY, x = bx + c, y = by + r;
-        if (x < nx && y < ny) put(oT + ((size_t)x * ny + y) * 8, r, c);
+        if (x < nx && y < ny) put(oT + ((size_t)x * py + y) * 8, r, c);
     }
 }
 
-// Interleaved copies from three slices on: a group of eight costs the same with
-// fewer, 36 us against 71 us planar for 3 x 301^2 x 257 (two planar slices cost
-// about as much as a group).  Their 16 planes are not taken for few planes of
-// a size where they would claim a good part of the memory.
-static bool use_interleaved(int nx, int ny, int nslices)
+// Whether the projector reads interleaved copies.  Eight slices and more do.  Fewer share
+// a group of eight, whose projection costs the same (us, interleaved | planar): 5 to 7
+// slices against two planar groups of four, 1024^2 x 360 604 | 1608; three slices
+// against two of two, 304^2 x 96 27 | 35, 1003^2 x 257 446 | 641; four slices against
+// one of four, 901^2 x 128 205 | 225, x 360 485 | 594, and at widths that are multiples
+// of 32, which make planar rows slower, 512^2 x 64 43 | 55.  The copies (16 planes
+// written, 2 us more than the planar transposition at 300^2, 11 at 800^2, 23 at 1024^2,
+// 55 at 2048^2) have to be earned by enough angles.  The 16 planes are not taken for
+// few planes of a size where they would claim a good part of the memory.
+static bool use_interleaved(int nx, int ny, int nslices, int nangles)
 {
-    return nslices >= 8 || (nslices >= 3 && (size_t)nx * ny <= ((size_t)1 << 26));
+    if (nslices >= 8) return true;
+    if (nslices < 3 || (size_t)nx * ny > ((size_t)1 << 26)) return false;
+    if (nslices >= 5) return nangles >= 16;
+    if (nslices == 3) return nangles >= 48;
+    return nangles >= ((nx | ny) % 32 ? 128 : 16);
 }
 
-size_t proj_scratch_bytes(int nx, int ny, int nslices)
+static size_t il_bytes(int nx, int ny, int nslices)
+{
+    const size_t pixels = (size_t)ny * il_pitch(nx) + (size_t)nx * il_pitch(ny);
+    return ((nslices + 7) / 8 * pixels + 1) * 8 * sizeof(float);
+}
+
+// of up to nslices planes: a last, smaller chunk may be the one that takes the copies
+size_t proj_scratch_bytes(int nx, int ny, int nslices, int nangles)
 {
     const size_t plane = (size_t)nx * ny * sizeof(float);
     if (nslices <= 0) return 16;
-    if (use_interleaved(nx, ny, nslices)) return 2 * (size_t)((nslices + 7) / 8) * 8 * plane + 8 * sizeof(float);
-    return (size_t)nslices * plane;
+    size_t bytes = 0;
+    for (int n = nslices < 8 ? 1 : nslices; n <= nslices; n++)
+        bytes = std::max(bytes, use_interleaved(nx, ny, n, nangles)
+                                    ? il_bytes(nx, ny, n)
+                                    : n * plane);
+    return bytes;
 }
 
 void stage_proj_images(ProjLaunch &pl, void *scratch, cudaStream_t st)
 {
     if (pl.nslices <= 0) return;
-    if (use_interleaved(pl.nx, pl.ny, pl.nslices)) {
+    if (use_interleaved(pl.nx, pl.ny, pl.nslices, pl.nangles)) {
         // the projector indexes a pixel of the interleaved copies in 32 bits
-        RAFT_CHECK((size_t)pl.nx * pl.ny <= 0xffffffffull, "projector: image plane above 2^32 pixels");
+        RAFT_CHECK(std::max((size_t)pl.ny * il_pitch(pl.nx), (size_t)pl.nx * il_pitch(pl.ny)) <= 0xffffffffull,
+                   "projector: image plane above 2^32 pixels");
         const int G = (pl.nslices + 7) / 8;
         float *il = (float *)scratch;
-        float *ilT = il + (size_t)G * 8 * pl.nx * pl.ny;
-        float *zero8 = ilT + (size_t)G * 8 * pl.nx * pl.ny;
+        float *ilT = il + (size_t)G * 8 * pl.ny * il_pitch(pl.nx);
+        float *zero8 = ilT + (size_t)G * 8 * pl.nx * il_pitch(pl.ny);
         count_launch();
         const unsigned bx = (pl.nx + 31) / 32, by = (pl.ny + 31) / 32;
         if ((long long)bx * by * G < 2 * 148)

@@ -241,11 +241,11 @@ int project_blocks_per_slice(int nrays, int nangles);
 // out[k][x][y] = in[k][y][x] for each of nslices planes.
 void launch_transpose(const float *in, float *out, int nx, int ny, int nslices, cudaStream_t st);
 
-// Scratch bytes the projector's re-laid-out images need for nslices planes.
-size_t proj_scratch_bytes(int nx, int ny, int nslices);
+// Scratch bytes the projector's re-laid-out images need for up to nslices planes.
+size_t proj_scratch_bytes(int nx, int ny, int nslices, int nangles);
 // Write the re-laid-out copies of pl.img into `scratch` (proj_scratch_bytes):
-// slice-interleaved groups of 8 (pl.il / pl.ilT) when there are 3 or more
-// planes, else a transposed copy (pl.imgT).  Issued on st.
+// slice-interleaved groups of 8 (pl.il / pl.ilT), or for few planes a transposed copy
+// (pl.imgT).  Issued on st.
 void stage_proj_images(ProjLaunch &pl, void *scratch, cudaStream_t st);
 
 // Flat/dark correction (and -log when is_log) of frames [nslices][nangles][nrays]
