@@ -148,7 +148,11 @@ const FilterPlan &cached_filter_plan(int device, int geometry, int ftype, int N,
 // ----------------------------------------------------------- host copies --
 void parallel_memcpy(void *dst, const void *src, size_t bytes)
 {
-    const size_t kMin = 8u << 20;
+    // a thread per 4 MB: chunks of the pipeline are a third of a call.  1024^2 x 900,
+    // 12 slices, lowpass: 4.9 ms in one chunk, 7.5 ms in three of 15 MB that one thread
+    // copied (a thread per 8 MB), 4.1 ms now; a thread per 2 MB gains more on large
+    // calls but loses a quarter on copies of 3 MB (4 x 512^2 x 360)
+    const size_t kMin = 4u << 20;
     unsigned hw = std::max(1u, std::thread::hardware_concurrency());
     unsigned nt = (unsigned)std::min<size_t>(std::min(8u, hw), bytes / kMin);
     if (nt <= 1) {
@@ -178,17 +182,19 @@ static bool is_pinned(const void *p)
     return at.type == cudaMemoryTypeHost;
 }
 
+// group: slices that the device takes together.
 template <class F>
-static void run_pipeline(DeviceState &ds, int nslices, int chunk, size_t in_ps, size_t out_ps,
+static void run_pipeline(DeviceState &ds, int nslices, int chunk, int group, size_t in_ps, size_t out_ps,
                          const void *host_in, void *host_out, F compute)
 {
     if (nslices <= 0) return;
     // page-locked caller buffers are transferred directly; pageable ones are
     // staged through the device's pinned buffers by host threads
     const bool pin_src = is_pinned(host_in), pin_dst = is_pinned(host_out);
-    // staging copies are host work that the device can hide: at least three
-    // chunks (of whole four-slice groups) where there are slices for them
-    if (!pin_src || !pin_dst) chunk = std::min(chunk, std::max(4, (nslices / 3 + 3) / 4 * 4));
+    // staging copies are host work that the device can hide: chunks of a third of the
+    // slices, rounded up to whole groups (two or three chunks).  Against one chunk of up
+    // to 32: FBP 1024^2 x 900, 8 slices 5.1 -> 3.6 ms, 16 8.2 -> 5.3, 32 14.8 -> 10.2
+    if (!pin_src || !pin_dst) chunk = std::min(chunk, std::max(group, (nslices / 3 + group - 1) / group * group));
     void *din[2], *dout[2], *pin[2] = {nullptr, nullptr}, *pout[2] = {nullptr, nullptr};
     for (int b = 0; b < 2; b++) {
         din[b] = ds.sino[b].get(in_ps * chunk);
@@ -405,7 +411,7 @@ void fbp_host_slab(const FbpConfig &cfg, int device, float *obj, const float *to
     const size_t out_ps = (size_t)fp.No * fp.No * sizeof(float);
     const int chunk = auto_chunk(nslices, in_ps, cfg.blocksize);
     void *rows = ds.il.get(fbp_ws_bytes(fp, chunk));
-    run_pipeline(ds, nslices, chunk, in_ps, out_ps, tomo, obj, [&](void *din, void *dout, int ns, cudaStream_t st) {
+    run_pipeline(ds, nslices, chunk, 4, in_ps, out_ps, tomo, obj, [&](void *din, void *dout, int ns, cudaStream_t st) {
         fbp_chunk(fp, tb, (const float *)din, (float *)dout, ns, rows, st, true);
     });
     check_device_flag(tb.err, "FBP");
@@ -429,7 +435,7 @@ void rotaxis_host_slab(int device, float *tomo, float axis_offset, int nrays, in
                                                 (double)axis_offset, 1.0);
     const size_t ps = (size_t)nangles * nrays * sizeof(float);
     const int chunk = auto_chunk(nslices, ps, blocksize);
-    run_pipeline(ds, nslices, chunk, ps, ps, tomo, tomo, [&](void *din, void *dout, int ns, cudaStream_t st) {
+    run_pipeline(ds, nslices, chunk, 4, ps, ps, tomo, tomo, [&](void *din, void *dout, int ns, cudaStream_t st) {
         FilterLaunch fl;
         fl.sino = (const float *)din;
         fl.out = dout;
@@ -509,13 +515,15 @@ void temfq_host_slab(const TemfqConfig &cfg, int device, float *obj, const float
 
 // ------------------------------------------------------------------ BST --
 // getBSTGPU (bst.cu:534-642): slices stream through the two-slot pipeline;
-// each chunk runs the three BST kernels (bst.cu in this library).
+// each chunk runs the BST kernels (bst.cu in this library).
 static int bst_chunk_slices(const BstPlanShape &sh, int nslices, int blocksize)
 {
-    // keep the per-chunk workspace near 4 GB (polar rows + crop columns)
+    // keep the per-chunk workspace near 4 GB (polar rows, grid), whole groups of the
+    // eight slices that share a grid point's geometry
     const size_t per = bst_workspace_bytes(sh, 1);
     int c = (int)std::max<size_t>(1, ((size_t)4 << 30) / std::max<size_t>(per, 1));
     c = std::min(c, 32);
+    if (c > 8) c -= c % 8;
     if (blocksize > 0) c = std::min(c, blocksize);
     return std::max(1, std::min(c, nslices));
 }
@@ -534,7 +542,7 @@ void bst_host_slab(const FbpConfig &cfg, int device, float *obj, const float *to
     const size_t out_ps = (size_t)cfg.nrays * cfg.nrays * sizeof(float);
     const int chunk = bst_chunk_slices(sh, nslices, cfg.blocksize);
     void *ws = ds.rows.get(bst_workspace_bytes(sh, chunk));
-    run_pipeline(ds, nslices, chunk, in_ps, out_ps, tomo, obj, [&](void *din, void *dout, int ns, cudaStream_t st) {
+    run_pipeline(ds, nslices, chunk, 4, in_ps, out_ps, tomo, obj, [&](void *din, void *dout, int ns, cudaStream_t st) {
         launch_bst(device, cfg, (const float *)din, (float *)dout, ns, ws, st);
     });
 }
@@ -567,7 +575,7 @@ void lowpass_host_slab(const FbpConfig &cfg, int device, float *tomo, int nslice
                                                 cfg.reg, 0.0, cfg.pixel_x);
     const size_t ps = (size_t)cfg.nangles * cfg.nrays * sizeof(float);
     const int chunk = auto_chunk(nslices, ps, cfg.blocksize);
-    run_pipeline(ds, nslices, chunk, ps, ps, tomo, tomo, [&](void *din, void *dout, int ns, cudaStream_t st) {
+    run_pipeline(ds, nslices, chunk, 4, ps, ps, tomo, tomo, [&](void *din, void *dout, int ns, cudaStream_t st) {
         FilterLaunch fl;
         fl.sino = (const float *)din;
         fl.out = dout;
@@ -600,7 +608,7 @@ void background_host_slab(int device, float *frames, const float *flat, const fl
     const size_t ps = (size_t)nangles * nrays * sizeof(float);
     const int chunk = auto_chunk(nslices, ps, blocksize);
     int s0 = 0;   // first slice of the chunk being computed (chunks run in order)
-    run_pipeline(ds, nslices, chunk, ps, ps, frames, frames, [&](void *din, void *dout, int ns, cudaStream_t st) {
+    run_pipeline(ds, nslices, chunk, 4, ps, ps, frames, frames, [&](void *din, void *dout, int ns, cudaStream_t st) {
         launch_background((const float *)din, (float *)dout, d_flat + (size_t)s0 * numflats * nrays,
                           d_dark + (size_t)s0 * nrays, nrays, nangles, ns, numflats, is_log, st);
         s0 += ns;
@@ -622,7 +630,13 @@ void radon_host_slab(int device, float *proj, const float *img, const float *ang
     const size_t out_ps = (size_t)nangles * nrays * sizeof(float);
     const int chunk = auto_chunk(nslices, std::max(in_ps, out_ps), 0);
     void *scratch = ds.imgT.get(proj_scratch_bytes(nx, ny, chunk, nangles));
-    run_pipeline(ds, nslices, chunk, in_ps, out_ps, img, proj, [&](void *din, void *dout, int ns, cudaStream_t st) {
+    // A chunk of four slices costs the projector as much as one of eight.  That hides behind
+    // the copies while it takes less than about half of their time (8 slices, chunks of
+    // eight | four: 1024^2 x 900 5.5 | 4.6 ms, 2048^2 x 900 16.1 | 17.1): 1.6 ps per pixel
+    // and angle against 16 bytes per pixel and sample at 8 GB/s.
+    const double pixels = (double)nx * ny, samples = (double)nangles * nrays;
+    const int group = pixels * nangles > 560.0 * (pixels + samples) ? 8 : 4;
+    run_pipeline(ds, nslices, chunk, group, in_ps, out_ps, img, proj, [&](void *din, void *dout, int ns, cudaStream_t st) {
         ProjLaunch pl;
         pl.img = (const float *)din;
         pl.out = (float *)dout;
