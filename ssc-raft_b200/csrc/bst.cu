@@ -34,7 +34,7 @@
 //                      grid point (square root, arc tangent, divisions) is worked
 //                      out once for up to eight slices;
 //   bst_gridrows_kernel  one grid row per CTA: inverse FFT along x, keeps the N
-//                      crop columns;
+//                      crop columns (small grids: bst_regrid_rows_kernel does both);
 //   bst_cols_kernel    two crop columns per CTA: inverse FFT along y, keeps
 //                      the N crop rows, scales.
 // This file is compiled with fast math, as the reference is, so the regrid
@@ -220,9 +220,23 @@ __device__ __forceinline__ float2 polar_value(const float2 *pol, const GridPoint
     return make_float2((i0.x * tf + i1.x * (1.f - tf)) * g.sgn, (i0.y * tf + i1.y * (1.f - tf)) * g.sgn);
 }
 
+// Conjugate of a grid point of one slice, or of its Hermitian part (m: the mirror image
+// through the origin).
+template <bool HALF>
+__device__ __forceinline__ float2 grid_value(const float2 *pol, const GridPoint &g, const GridPoint &m)
+{
+    const float2 u = polar_value(pol, g);
+    if constexpr (HALF) {
+        const float2 v = polar_value(pol, m);
+        return make_float2(0.5f * (u.x + v.x), 0.5f * (v.y - u.y));   // conj of (u + conj v) / 2
+    } else {
+        return make_float2(u.x, -u.y);
+    }
+}
+
 constexpr int kRegridSlices = 8;
 // One thread per grid point of rows 0 .. H-1, for up to eight slices: the point
-// and, on the half grid, its mirror image through the origin.  The arithmetic of the two positions
+// and, on the half grid, its mirror image.  The arithmetic of the two positions
 // (about 200 instructions) is paid once per eight slices; with one grid row and
 // slice per CTA, transformed in place, the kernel was bound by it: 413 us per
 // 2048^2 x 1800 slice (6144 x 6144 points).
@@ -240,15 +254,29 @@ __global__ void __launch_bounds__(256) bst_regrid_kernel(const BstArgs p, int ns
     const float2 *pol = p.polar + b0 * per;
     float2 *out = p.grid + b0 * plane + (size_t)Y * S + X;
 #pragma unroll 4
-    for (int b = b0; b < b1; b++, pol += per, out += plane) {
-        const float2 u = polar_value(pol, g);
-        if constexpr (HALF) {
-            const float2 v = polar_value(pol, m);
-            *out = make_float2(0.5f * (u.x + v.x), 0.5f * (v.y - u.y));   // conj of (u + conj v) / 2
-        } else {
-            *out = make_float2(u.x, -u.y);
-        }
+    for (int b = b0; b < b1; b++, pol += per, out += plane) *out = grid_value<HALF>(pol, g, m);
+}
+
+// One grid row of one slice per CTA, interpolated straight into shared memory and
+// transformed: small grids, where the geometry per slice costs less than another
+// kernel and the pass through memory (fuse_regrid).  T is not the polar rows' buffer
+// here: other CTAs still read them.
+template <bool HALF>
+__global__ void __launch_bounds__(512) bst_regrid_rows_kernel(const BstArgs p)
+{
+    extern __shared__ float2 sm_bst[];
+    const int slice = blockIdx.y, Y = blockIdx.x, S = p.S;
+    const float2 *pol = p.polar + (size_t)slice * 2 * p.A * p.Lh;
+    for (int X = threadIdx.x; X < S; X += blockDim.x) {
+        const GridPoint g = grid_point(p, X, Y);
+        GridPoint m{};
+        if constexpr (HALF) m = grid_point(p, X ? S - X : 0, Y ? S - Y : 0);
+        sm_bst[X] = grid_value<HALF>(pol, g, m);
     }
+    __syncthreads();
+    const float2 *r = bst_fft<0>(sm_bst, sm_bst + fft_plan_span(p.pS), p.pS);
+    float2 *trow = p.T + ((size_t)slice * p.H + Y) * p.N;
+    for (int i = threadIdx.x; i < p.N; i += blockDim.x) trow[i] = r[p.off + i];
 }
 
 // T = the forward transform of the conjugated rows: conj of their inverse transform
@@ -550,8 +578,15 @@ static void launch_bst_rows(const BstArgs &a, const BstCore &c, int nslices, int
     RAFT_CUDA(cudaGetLastError());
 }
 
+// Grids without a compiled length of up to 2.5 million points in all slices are
+// interpolated and transformed in one kernel.  Another kernel costs 2 - 5 us, geometry per
+// slice about 1 us per 10^5 points: us, split | fused, 128^2 x 360 (256 x 256
+// points), 2 slices 33 | 29, 250^2 x 90 (500 x 500), 4 slices 46 | 44, 300^2 x 90 (900 x 900),
+// 3 slices 71 | 70, 12 slices 146 | 158.
+static bool fuse_regrid(int S, int nslices) { return (double)nslices * S * S <= 2.5e6; }
+
 template <int NF>
-static void launch_bst_grid(const BstArgs &a, const BstCore &c, int nslices, int threads, size_t sm2, cudaStream_t st)
+static void launch_bst_grid(BstArgs a, const BstCore &c, int nslices, int threads, size_t sm2, cudaStream_t st)
 {
     static thread_local int configured = -1;
     int dev = 0;
@@ -563,14 +598,27 @@ static void launch_bst_grid(const BstArgs &a, const BstCore &c, int nslices, int
                                        (int)kBstSmemMax));
         RAFT_CUDA(cudaFuncSetAttribute(bst_cols_kernel<NF, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        (int)kBstSmemMax));
+        if (NF == 0) {
+            RAFT_CUDA(cudaFuncSetAttribute(bst_regrid_rows_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                           (int)kBstSmemMax));
+            RAFT_CUDA(cudaFuncSetAttribute(bst_regrid_rows_kernel<false>,
+                                           cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kBstSmemMax));
+        }
         configured = dev;
     }
-    const dim3 grid((c.S + 31) / 32, (a.H + 7) / 8, (nslices + kRegridSlices - 1) / kRegridSlices);
-    if (c.half_grid) bst_regrid_kernel<true><<<grid, dim3(32, 8), 0, st>>>(a, nslices);
-    else bst_regrid_kernel<false><<<grid, dim3(32, 8), 0, st>>>(a, nslices);
-    RAFT_CUDA(cudaGetLastError());
-    count_launch();
-    bst_gridrows_kernel<NF><<<dim3(a.H, nslices), threads, sm2, st>>>(a);
+    if (NF == 0 && fuse_regrid(c.S, nslices)) {
+        a.T = a.grid;
+        if (c.half_grid) bst_regrid_rows_kernel<true><<<dim3(a.H, nslices), threads, sm2, st>>>(a);
+        else bst_regrid_rows_kernel<false><<<dim3(a.H, nslices), threads, sm2, st>>>(a);
+    } else {
+        a.T = a.polar;   // the polar rows are read before the grid rows are transformed
+        const dim3 grid((c.S + 31) / 32, (a.H + 7) / 8, (nslices + kRegridSlices - 1) / kRegridSlices);
+        if (c.half_grid) bst_regrid_kernel<true><<<grid, dim3(32, 8), 0, st>>>(a, nslices);
+        else bst_regrid_kernel<false><<<grid, dim3(32, 8), 0, st>>>(a, nslices);
+        RAFT_CUDA(cudaGetLastError());
+        count_launch();
+        bst_gridrows_kernel<NF><<<dim3(a.H, nslices), threads, sm2, st>>>(a);
+    }
     RAFT_CUDA(cudaGetLastError());
     count_launch();
     if (c.half_grid) bst_cols_kernel<NF, true><<<dim3((c.N + 1) / 2, nslices), threads, sm2, st>>>(a);
@@ -587,7 +635,7 @@ void bst_run(int device, const BstCore &c, const float *d_tomo, float *d_obj, in
     BstArgs a;
     a.tomo = d_tomo;
     a.polar = (float2 *)workspace;
-    a.T = a.polar;   // the polar rows are read before the grid rows are transformed
+    a.T = nullptr;   // launch_bst_grid
     a.grid = (float2 *)((char *)workspace + bst_polar_bytes(c.A, c.Lh, c.rows(), c.N, nslices));
     a.obj = d_obj;
     a.G = c.G;
