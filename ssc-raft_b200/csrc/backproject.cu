@@ -299,15 +299,7 @@ __device__ __forceinline__ bool bp_tile(const BpArgs &p, const int AB, const int
                         const float m = __fadd_rn(v, MAGIC);
                         const unsigned k = min((unsigned)(__float_as_int(m) - 0x4B400000), (unsigned)(W - 1));
                         const float f = __fsub_rn(v, __fsub_rn(m, MAGIC));
-                        if constexpr (IL && STORE == STORE_PAIR_F32) {
-                            // bin k: (mid, dif) of slices 0..3 in 32 bytes
-                            const float4 u0 = reinterpret_cast<const float4 *>(w)[2 * k];
-                            const float4 u1 = reinterpret_cast<const float4 *>(w)[2 * k + 1];
-                            acc[0][j][i] += fmaf(f, u0.y, u0.x);
-                            acc[1][j][i] += fmaf(f, u0.w, u0.z);
-                            acc[2][j][i] += fmaf(f, u1.y, u1.x);
-                            acc[3][j][i] += fmaf(f, u1.w, u1.z);
-                        } else if constexpr (IL) {
+                        if constexpr (IL) {
                             // bin k: bf16 (mid, dif) pairs of slices 0..3 in 16 bytes;
                             // value = mid + f dif per slice, two slices per instruction
                             const uint4 u = reinterpret_cast<const uint4 *>(w)[k];
@@ -715,8 +707,12 @@ static void launch_bp_cfg(const BpArgs &a, BpTune t, cudaStream_t st)
     case 1: launch_bp_s<GEOM, STORE, 1>(a, t.AB, st); break;
     case 2: launch_bp_s<GEOM, STORE, 2>(a, t.AB, st); break;
     default:
-        if (a.il) launch_bp_s<GEOM, STORE, 4, true>(a, t.AB, st);
-        else launch_bp_s<GEOM, STORE, 4>(a, t.AB, st);
+        if constexpr (STORE != STORE_PAIR_F32)   // pairs of floats are planar
+            if (a.il) {
+                launch_bp_s<GEOM, STORE, 4, true>(a, t.AB, st);
+                break;
+            }
+        launch_bp_s<GEOM, STORE, 4>(a, t.AB, st);
         break;
     }
 }
@@ -725,7 +721,10 @@ static void launch_bp_any(const BpArgs &a, int geometry, int store, BpTune t, cu
 {
     switch (geometry) {
     case GEOM_FBP_REF: launch_bp_cfg<GEOM_FBP_REF, STORE_F32>(a, t, st); break;
-    case GEOM_EM_REF: launch_bp_cfg<GEOM_EM_REF, STORE_F32>(a, t, st); break;
+    case GEOM_EM_REF:   // rows of EM are interleaved by slice
+        RAFT_CHECK(a.il && t.S == 4, "backprojector: EM rows are interleaved");
+        launch_bp_s<GEOM_EM_REF, STORE_F32, 4, true>(a, t.AB, st);
+        break;
     default:
         if (store == STORE_PAIR_BF16) launch_bp_cfg<GEOM_FBP_LIN, STORE_PAIR_BF16>(a, t, st);
         else launch_bp_cfg<GEOM_FBP_LIN, STORE_PAIR_F32>(a, t, st);

@@ -574,13 +574,16 @@ template <int NP, bool CONV>
 static void launch_fixed_np(const FilterPlan &plan, const FilterLaunch &fl, const PackArgs &pk, int nsl,
                             cudaStream_t st)
 {
-    const bool f32 = fl.store == STORE_F32;
-    if (fl.interleaved) {
-        if (f32) launch_fixed_one<NP, true, true, CONV>(plan, fl, pk, nsl, st);
-        else launch_fixed_one<NP, true, false, CONV>(plan, fl, pk, nsl, st);
+    if (fl.store == STORE_F32) {
+        if (fl.interleaved) launch_fixed_one<NP, true, true, CONV>(plan, fl, pk, nsl, st);
+        else launch_fixed_one<NP, false, true, CONV>(plan, fl, pk, nsl, st);
+        return;
+    }
+    if constexpr (CONV) {
+        RAFT_CHECK(false, "filter: convolution rows are single floats");   // conv_length
     } else {
-        if (f32) launch_fixed_one<NP, false, true, CONV>(plan, fl, pk, nsl, st);
-        else launch_fixed_one<NP, false, false, CONV>(plan, fl, pk, nsl, st);
+        if (fl.interleaved) launch_fixed_one<NP, true, false, false>(plan, fl, pk, nsl, st);
+        else launch_fixed_one<NP, false, false, false>(plan, fl, pk, nsl, st);
     }
 }
 

@@ -1020,7 +1020,8 @@ int launch_wgrad_tc9(const CUtensorMap &m0, const CUtensorMap &m1, const CUtenso
     return cudaGetLastError() == cudaSuccess ? 0 : 1;
 }
 
-// dw[co][r] += sum over splits of part[split][r][co], r = tap * Cin + ci < rows.
+// dw[co][r] += sum over splits of part[split][r][co], r = tap * Cin + ci < rows
+// (a multiple of 4: Cin is one of 32).
 // A block takes four r and 32 co; its eight warps share the splits (warp w sums
 // w, w + 8, ...), whose sums are added in warp order.  With one thread walking all
 // splits of an element, 32 -> 32 channels (9216 elements, 148 splits) had 36
@@ -1038,7 +1039,7 @@ __global__ void __launch_bounds__(256) wgrad_reduce_kernel(const float *__restri
     for (int sp = warp; sp < splits; sp += 8)
 #pragma unroll
         for (int q = 0; q < 4; q++)
-            if (r0 + q < rows) acc[q] += __ldcs(src + sp * stride + (size_t)q * Cout);
+            acc[q] += __ldcs(src + sp * stride + (size_t)q * Cout);
 #pragma unroll
     for (int q = 0; q < 4; q++) red[warp][q][lane] = acc[q];
     __syncthreads();
@@ -1047,7 +1048,7 @@ __global__ void __launch_bounds__(256) wgrad_reduce_kernel(const float *__restri
         float sum = 0.f;
 #pragma unroll
         for (int w = 0; w < 8; w++) sum += red[w][q][co];
-        if (r0 + q < rows) dw[(size_t)(c0 + co) * rows + r0 + q] += sum;
+        dw[(size_t)(c0 + co) * rows + r0 + q] += sum;
     }
 }
 

@@ -8,7 +8,8 @@ the FP64 oracle: lowpass <= 3e-6 rel-L2 on uniform noise in [1, 2], whose filter
 rows keep a fixed share of the input's norm (two FP32 transforms of M points with
 an error of about 1.2e-7 sqrt(log2 M) each, times three; measured <= 9.3e-7, with
 Bluestein's algorithm <= 1.4e-6), and the kernels compiled for the transform length
-against the generic one, bit for bit, for every row format."""
+against the generic one, bit for bit, on planar and interleaved rows (single floats: the
+nearest-sample operator has no other row format)."""
 import ctypes
 import os
 
@@ -43,8 +44,8 @@ def test_lowpass_vs_oracle(oracle, N, pad, ftype):
 
 
 @pytest.mark.parametrize("N,pad", [(257, 1), (251, 1), (341, 2), (1023, 1)])
-@pytest.mark.parametrize("geometry,store,tune", [(0, 0, None), (0, 0, "2,16"), (1, 1, None), (1, 1, "2,16"), (1, 2, None)])
-def test_compiled_length_equals_generic(N, pad, geometry, store, tune):
+@pytest.mark.parametrize("tune", [None, "2,16"])     # interleaved rows, planar rows
+def test_compiled_length_equals_generic(N, pad, tune):
     import torch
     from sscRaft.rafttypes import _ptr, libraft
     A, n = 37, 5
@@ -60,8 +61,7 @@ def test_compiled_length_equals_generic(N, pad, geometry, store, tune):
         for fixed in (1, 0):
             libraft.raft_filter_set_fixed(fixed)
             out = torch.empty((n, N, N), device="cuda")
-            assert libraft.raft_fbp_device(0, _p(out), _p(sino), _ptr(ang), _ptr(pf), _ptr(pi), geometry, store,
-                                           None) == 0
+            assert libraft.raft_fbp_device(0, _p(out), _p(sino), _ptr(ang), _ptr(pf), _ptr(pi), 0, 0, None) == 0
             outs.append(out)
     finally:
         libraft.raft_filter_set_fixed(1)

@@ -3,8 +3,8 @@
 the per-tap tiles (<= 2e-3), at heights that leave a part of a 2- or 4-row tile, widths
 around its 128 pixels, several images, and the split output of the data gradient.
 The weight gradient's reduction over splits, whose eight warps take them in turn: one
-k-block (one split), fewer splits than warps, and 9 Cin rows that are no multiple of
-the block's four, against the oracle (<= 1e-4, as in test_gpu_unet_tc.py)."""
+k-block (one split) and fewer splits than warps, against the oracle (<= 1e-4, as in
+test_gpu_unet_tc.py)."""
 import numpy as np
 import pytest
 

@@ -63,7 +63,7 @@ def test_layers_on_two_streams(own):
     assert not bad, bad
 
 
-def test_two_short_workspaces_are_refused():
+def test_a_short_workspace_is_refused():
     import torch
     from sscRaft import warmstart as ws
     from sscRaft.rafttypes import libraft
