@@ -725,6 +725,14 @@ def peaks():
     return 6650.0, 1965.0, "fallback"
 
 
+# Bytes of shared memory that the run kernel reads per update, averaged over [0, pi): four
+# pixels in a row share 2, 3, 3 or 4 samples where the detector position moves by up to
+# 1/3, 1/2, 2/3 and 1/sqrt(2) bins per pixel; linear interpolation reads 4, 5, 4 or 6.
+_RUN_SHARE = np.diff(np.degrees(np.arcsin([0, 1 / 3, 1 / 2, 2 / 3, 0.5 ** 0.5]))) / 45.0
+RUN_BYTES = float(_RUN_SHARE @ [2, 3, 3, 4])
+RUN_BYTES_LINEAR = float(_RUN_SHARE @ [4, 5, 4, 6])
+
+
 def gather_peak_gups(store_bytes, ops, sm_mhz, n_sm=148):
     """Backprojection gather roofline: SMs x clock x min(smem bytes/clk / bytes
     per update, FP32 lanes / FP32 ops per update)."""
@@ -942,10 +950,10 @@ def run_ours(args):
     alg_bytes = chunk * N_ANGLES * reach * 4 + chunk * N_RAYS * N_RAYS * 4
     sm_mhz = (clocks or {}).get("sm_mhz") or sm_max
     gups_bp = upd_per_launch / bp_avg_s / 1e9
-    peak_gups = gather_peak_gups(4, 4, sm_mhz)
-    # linear f32: two samples, 8 B + 5 FP32 ops per update; bf16 pairs on slice-interleaved rows:
-    # 4 B + 4 ops (two FP32, two integer to unpack the pair)
-    for name, (g, s, bytes_upd, ops) in (("linear_fp32", (1, 1, 8, 5)), ("linear_bf16", (1, 2, 4, 4))):
+    peak_gups = gather_peak_gups(RUN_BYTES, 1, sm_mhz)
+    # bf16 pairs: as many elements, 4 ops (two FP32, two integer to unpack the pair)
+    for name, (g, s, bytes_upd, ops) in (("linear_fp32", (1, 1, RUN_BYTES_LINEAR, 2)),
+                                         ("linear_bf16", (1, 2, RUN_BYTES, 4))):
         _, _, vms, vn = profile_bp(g, s)
         vg = upd_per_launch / (vms / vn / 1e3) / 1e9
         pk = gather_peak_gups(bytes_upd, ops, sm_mhz)
@@ -993,9 +1001,10 @@ def run_ours(args):
                          "kernel": "bp_run_kernel<nearest,f32,16 slices per thread>",
                          "kernel_ms_per_launch": bp_avg_s * 1e3,
                          "updates_per_launch": upd_per_launch,
-                         "peak_def": "148 SMs x SM clock (median sampled) x 32 updates/clk: 128 B/clk of "
-                                     "shared-memory data pipe / 4 B per update (one sample read per update; "
-                                     "the run kernel reads 2.6 B, so frac can pass 1)",
+                         "peak_def": "148 SMs x SM clock (median sampled) x 48.5 updates/clk: 128 B/clk of "
+                                     "shared-memory data pipe / 2.64 B per update (what the run kernel reads, "
+                                     "averaged over the angles; its spills share the pipe, 87 % of whose "
+                                     "wavefronts are used)",
                          "sm_mhz": sm_mhz,
                          "traffic": None,
                          "traffic_source": "not captured at this size",
@@ -1003,7 +1012,7 @@ def run_ours(args):
                          "hbm": {"achieved_gbs": alg_bytes / bp_avg_s / 1e9, "peak_gbs": hbm_peak,
                                  "frac": alg_bytes / bp_avg_s / 1e9 / hbm_peak, "peak_kind": peak_kind}},
             "gather_roofline": {"achieved_gups": gups_bp, "peak_gups": peak_gups, "frac": gups_bp / peak_gups,
-                                "bytes_per_update": 4, "fp32_ops_per_update": 4, "sm_mhz": sm_mhz},
+                                "bytes_per_update": RUN_BYTES, "fp32_ops_per_update": 1, "sm_mhz": sm_mhz},
             "kernel_ms": {"filter_per_launch": f_ms / max(1, f_n), "bp_per_launch": bp_ms / max(1, bp_n),
                           "launches_per_step": {"filter": f_n, "bp": bp_n}},
             "variants": variants,

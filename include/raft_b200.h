@@ -283,8 +283,9 @@ int raft_unet_conv_fwd(const void *x0, int C0, const void *x1, int C1, const voi
  * or W dividing 128), mma.sync kernel otherwise (default); 1 = mma.sync kernel only;
  * 2 = tcgen05 kernel only (other shapes fail). */
 int raft_unet_set_conv_path(int path);
-/* tcgen05 convolution of the 32 -> 32 channel layers (W >= 128): 1 = halo tiles (one input
- * box per 32-channel chunk serves all nine taps; default), 0 = one input box per tap. */
+/* tcgen05 convolution of layers with few channels (W >= 128; up to 96 -> 32, 32 -> 64 or 96):
+ * 1 = halo tiles (one input box per 32-channel chunk serves all nine taps; default), 0 = one
+ * input box per tap. */
 int raft_unet_set_conv_halo(int on);
 /* tcgen05 weight gradient (W a multiple of 64; Cout 32, 64, 128 or 256; other shapes and
  * raft_unet_set_conv_path(1) use the mma.sync kernel): 1 = for Cout <= 128 one CTA per

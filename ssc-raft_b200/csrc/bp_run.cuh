@@ -1,6 +1,6 @@
-// bp_run.cuh -- the four-slice backprojector on slice-interleaved rows, with
-// each thread's pixels arranged as runs along the image axis on which the
-// detector coordinate moves slowest (included by backproject.cu).
+// bp_run.cuh -- the backprojector whose threads' pixels are runs along the image
+// axis on which the detector coordinate moves slowest: 16, 8 or 4 slices per thread
+// on slice-interleaved rows, or one on plain rows (included by backproject.cu).
 //
 // What bounds it, and why runs.  A gather of one 4-byte sample per
 // (voxel, angle) is limited by the 128 B/clk shared-memory pipe to 32 updates
@@ -8,10 +8,12 @@
 // (pixel, angle) ran at 87-90 % of that.  But at every angle one image axis has
 // |dt/dx| <= 1/sqrt(2) bins per pixel, so four neighbouring pixels along it fall
 // into two (|dt/dx| <= 1/3), three or at most four bins: the thread loads those
-// bins once and adds the right one to each pixel.  That is 2.6 instead of 4
+// bins once and adds the right one to each pixel.  That is 2.64 instead of 4
 // shared-memory bytes per update averaged over [0, pi); neighbouring pixels of
 // a run start in one of only two bins (slope classes below), so the choice is
-// one compare and two predicated two-lane adds per bin.  Position and rounding
+// one compare and one select per two slices.  16 x 2048^2 x 900, nearest: 87 % of
+// the pipe's wavefronts (80 % shared memory, most of the rest the spills of the
+// sixteen-slice form), 2.47 instructions per clock.  Position and rounding
 // are computed two pixels per instruction.  The bin of every pixel is still
 // computed by itself with the single-pixel kernel's expressions, and the order
 // of the additions over angles is the same: the images are bit for bit those of

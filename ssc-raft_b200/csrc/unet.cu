@@ -816,7 +816,7 @@ int raft_unet_set_conv_path(int path)
     return 0;
 }
 
-// Halo tiles of the tcgen05 convolution for its 32 -> 32 channel layers (1, the
+// Halo tiles of the tcgen05 convolution for layers with few channels (1, the
 // default) or the per-tap operand tiles for every layer (0).
 int raft_unet_set_conv_halo(int on)
 {
