@@ -779,16 +779,19 @@ static int forced_run()
 // are 32 x 32 pixels (run kernel) or 64 x 32 (single-pixel kernel), times `slices`.
 // Fitted to the times of 400 - 2100 launches per row (96^2 - 2048^2 pixels, 48 - 1024
 // angles over [0, pi), 1 - 32 slices); the fit is off by 1 - 3 % (root mean square).
+// `turn`: a change of the run axis with its classes of slopes, of which [0, pi) has two
+// (from scans over 2 pi, which have four: 8 x 700^2 x 120 nearest, single-pixel 121, run
+// 148 us for the whole pass).
 struct BpCost {
     int slices, width, resident;
-    float fixed[6], angle[6];
-    double time(int No, int nslices, int nangles) const
+    float fixed[6], angle[6], turn;
+    double time(int No, int nslices, int nangles, int turns) const
     {
         const long long blocks =
             (long long)((No + width - 1) / width) * ((No + 31) / 32) * ((nslices + slices - 1) / slices);
         const long long wave = 148LL * resident, before = (blocks - 1) / wave;
         const int last = (int)((blocks - before * wave + 147) / 148);
-        auto t = [&](int k) { return fixed[k] + (double)angle[k] * nangles; };
+        auto t = [&](int k) { return fixed[k] + (double)angle[k] * nangles + (double)turn * std::max(0, turns - 2); };
         return (double)before * t(resident) + t(last - 1);
     }
 };
@@ -802,46 +805,45 @@ enum { BP_SINGLE = 0, BP_SINGLE1, BP_SINGLE4, BP_ONE, BP_RUN4, BP_RUN8, BP_RUN16
 // accumulators and for the classes of slopes, and every grid pays for its last wave.
 static const BpCost kBpCost[4][BP_FORMS] = {
     // nearest sample, bins of unit width
-    {{4, 64, 3, {-1.2f, -0.3f, 0.5f, 2.3f}, {0.267f, 0.347f, 0.465f, 0.448f}},
+    {{4, 64, 3, {-1.2f, -0.3f, 0.5f, 2.3f}, {0.267f, 0.347f, 0.465f, 0.448f}, 0.f},
      {},
      {},
-     {1, 32, 4, {5.1f, 5.6f, 7.2f, 8.6f, 10.0f}, {0.071f, 0.101f, 0.141f, 0.185f, 0.164f}},
-     {4, 32, 3, {6.5f, 7.8f, 9.9f, 11.6f}, {0.115f, 0.174f, 0.25f, 0.223f}},
-     {8, 32, 2, {10.9f, 12.4f, 15.2f}, {0.155f, 0.255f, 0.232f}},
-     {16, 32, 2, {21.1f, 22.7f, 26.7f}, {0.3f, 0.499f, 0.449f}}},
+     {1, 32, 4, {5.1f, 5.6f, 7.2f, 8.6f, 10.0f}, {0.071f, 0.101f, 0.141f, 0.185f, 0.164f}, 4.8f},
+     {4, 32, 3, {6.5f, 7.8f, 9.9f, 11.6f}, {0.115f, 0.174f, 0.25f, 0.223f}, 4.6f},
+     {8, 32, 2, {10.9f, 12.4f, 15.2f}, {0.155f, 0.255f, 0.232f}, 5.5f},
+     {16, 32, 2, {21.1f, 22.7f, 26.7f}, {0.3f, 0.499f, 0.449f}, 7.2f}},
     // nearest sample, other bins (EM)
-    {{4, 64, 3, {-2.2f, -0.3f, 0.1f, 2.3f}, {0.247f, 0.333f, 0.458f, 0.443f}},
+    {{4, 64, 3, {-2.2f, -0.3f, 0.1f, 2.3f}, {0.247f, 0.333f, 0.458f, 0.443f}, 0.f},
      {},
      {},
-     {1, 32, 4, {4.7f, 5.2f, 6.1f, 7.6f, 9.1f}, {0.073f, 0.106f, 0.152f, 0.199f, 0.177f}},
-     {4, 32, 3, {6.0f, 7.1f, 8.5f, 10.8f}, {0.12f, 0.185f, 0.27f, 0.24f}},
-     {8, 32, 2, {10.0f, 11.6f, 14.7f}, {0.157f, 0.258f, 0.233f}},
-     {16, 32, 2, {18.1f, 21.3f, 25.1f}, {0.302f, 0.494f, 0.448f}}},
+     {1, 32, 4, {4.7f, 5.2f, 6.1f, 7.6f, 9.1f}, {0.073f, 0.106f, 0.152f, 0.199f, 0.177f}, 4.8f},
+     {4, 32, 3, {6.0f, 7.1f, 8.5f, 10.8f}, {0.12f, 0.185f, 0.27f, 0.24f}, 4.6f},
+     {8, 32, 2, {10.0f, 11.6f, 14.7f}, {0.157f, 0.258f, 0.233f}, 5.5f},
+     {16, 32, 2, {18.1f, 21.3f, 25.1f}, {0.302f, 0.494f, 0.448f}, 7.2f}},
     // linear interpolation, BF16 pairs
-    {{4, 64, 3, {-2.0f, -0.9f, -0.7f, 1.7f}, {0.445f, 0.579f, 0.827f, 0.724f}},
+    {{4, 64, 3, {-2.0f, -0.9f, -0.7f, 1.7f}, {0.445f, 0.579f, 0.827f, 0.724f}, 0.f},
      {},
      {},
-     {1, 32, 3, {5.7f, 6.1f, 7.0f, 9.5f}, {0.078f, 0.129f, 0.19f, 0.171f}},
-     {4, 32, 3, {7.2f, 8.2f, 9.5f, 10.9f}, {0.163f, 0.282f, 0.418f, 0.382f}},
-     {8, 32, 2, {12.9f, 14.4f, 15.6f}, {0.23f, 0.431f, 0.403f}},
+     {1, 32, 3, {5.7f, 6.1f, 7.0f, 9.5f}, {0.078f, 0.129f, 0.19f, 0.171f}, 3.9f},
+     {4, 32, 3, {7.2f, 8.2f, 9.5f, 10.9f}, {0.163f, 0.282f, 0.418f, 0.382f}, 3.7f},
+     {8, 32, 2, {12.9f, 14.4f, 15.6f}, {0.23f, 0.431f, 0.403f}, 5.6f},
      {}},
     // linear interpolation, FP32 (the single-pixel kernel: planar pairs; two slices per
     // block, or what was tuned: one, two or four)
-    {{2, 64, 4, {-2.4f, -1.6f, -0.7f, -0.3f, 2.5f}, {0.404f, 0.462f, 0.587f, 0.751f, 0.654f}},
-     {1, 64, 5, {-2.4f, -1.9f, -1.1f, -1.0f, -1.0f, 2.2f}, {0.209f, 0.285f, 0.397f, 0.524f, 0.646f, 0.579f}},
-     {4, 64, 3, {-2.7f, -0.4f, 0.4f, 2.8f}, {0.685f, 0.791f, 0.993f, 0.93f}},
+    {{2, 64, 4, {-2.4f, -1.6f, -0.7f, -0.3f, 2.5f}, {0.404f, 0.462f, 0.587f, 0.751f, 0.654f}, 0.f},
+     {1, 64, 5, {-2.4f, -1.9f, -1.1f, -1.0f, -1.0f, 2.2f}, {0.209f, 0.285f, 0.397f, 0.524f, 0.646f, 0.579f}, 0.f},
+     {4, 64, 3, {-2.7f, -0.4f, 0.4f, 2.8f}, {0.685f, 0.791f, 0.993f, 0.93f}, 0.f},
      {},
-     {4, 32, 3, {7.6f, 8.1f, 9.9f, 11.2f}, {0.165f, 0.29f, 0.429f, 0.39f}},
-     {8, 32, 2, {12.8f, 14.2f, 15.0f}, {0.238f, 0.447f, 0.416f}},
+     {4, 32, 3, {7.6f, 8.1f, 9.9f, 11.2f}, {0.165f, 0.29f, 0.429f, 0.39f}, 3.6f},
+     {8, 32, 2, {12.8f, 14.2f, 15.0f}, {0.238f, 0.447f, 0.416f}, 5.3f},
      {}},
 };
 constexpr double kNextLaunch = 5.0;   // a further launch of the same call (us)
 constexpr int kRunMinAngles = 48;     // below, the fit does not hold and nothing is gained
 
-// The run kernel's rule on positions needs pixels as wide as detector bins.  Turning
-// the accumulators costs about as much as three angles, so angle lists that change
-// the run axis more often than every 16 angles (scans in golden-ratio order) keep
-// the single-pixel kernel.
+// The run kernel's rule on positions needs pixels as wide as detector bins.  Angle
+// lists that change the run axis more often than every 16 angles (scans in
+// golden-ratio order) keep the single-pixel kernel.
 static bool run_possible(const BpGeo &g, int geometry)
 {
     if (geometry == GEOM_EM_REF) return g.dxy == g.dt;
@@ -874,7 +876,7 @@ BpSplit bp_split(const BpGeo &g, int geometry, int store, int No, int nslices, i
     }
     if (nangles < kRunMinAngles || turns > nangles / 16 + 2) return best;
     const BpCost *cost = kBpCost[f32 ? 3 : bf16 ? 2 : (geometry == GEOM_EM_REF || g.dt != 1.f) ? 1 : 0];
-    auto form_time = [&](int form, int slices) { return cost[form].time(No, slices, nangles); };
+    auto form_time = [&](int form, int slices) { return cost[form].time(No, slices, nangles, turns); };
     double t_best = form_time(BP_SINGLE, nslices);
     if (f32 && nslices >= 8)   // tuned
         t_best = std::min({t_best, form_time(BP_SINGLE1, nslices), form_time(BP_SINGLE4, nslices)});

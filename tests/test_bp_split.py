@@ -50,6 +50,17 @@ def test_every_slice_is_taken_once_and_by_a_form_that_exists(geometry, store):
         ({"g16"} if geometry != 1 else set())
 
 
+@pytest.mark.parametrize("geometry,store,N,A,n,single,run", [
+    (0, 0, 700, 120, 8, 121, 148), (0, 0, 384, 60, 2, 37, 46), (0, 0, 200, 60, 8, 38, 46), (0, 0, 700, 60, 1, 50, 58),
+    (1, 1, 200, 60, 1, 33, 49), (1, 1, 700, 60, 16, 187, 233), (1, 1, 1501, 60, 8, 435, 514)])
+def test_scans_over_two_pi_count_their_turns(geometry, store, N, A, n, single, run):
+    """Few angles over 2 pi (four changes of the run axis instead of two): whole passes
+    measured with the single-pixel and the run kernel (us)."""
+    assert single < run
+    s = _split(N, A, n, geometry, store, angles=np.arange(A) * (2 * np.pi / A))
+    assert s == [0, 0, 0, -(-n // 4), 0], s
+
+
 def test_where_the_run_kernel_does_not_apply():
     k = np.arange(300)
     assert _split(512, 300, 8, angles=(k * 2.3999632) % np.pi) == [0, 0, 0, 2, 0]      # turns too often
