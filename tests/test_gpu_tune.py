@@ -78,3 +78,26 @@ def test_em_shapes_bit_identical(restore_env):
         outs[c] = obj
     for c in CANDIDATES[1:] + [None]:
         assert torch.equal(outs[c], outs[CANDIDATES[0]]), c
+
+
+def test_one_slice_after_a_tuned_batch(restore_env):
+    """A shape tuned on a batch may take four slices per block; one or two slices do not
+    use it, and give the batch's bits."""
+    import torch
+    from sscRaft.rafttypes import _ptr, libraft
+    os.environ.pop("RAFT_BP_TUNE", None)
+    N, A, n = 300, 40, 32                 # below 48 angles: the single-pixel kernel, planar FP32 pairs
+    ang = (np.arange(A) * (np.pi / A)).astype(np.float32)
+    sino = torch.rand((n, A, N), generator=torch.Generator(device="cuda").manual_seed(9), device="cuda")
+    pf = np.array([0, 0, 1, 0, 1, 1, 0.5], np.float32)
+
+    def run(k0, k1):
+        x = sino[k0:k1].contiguous()
+        out = torch.empty((k1 - k0, N, N), device="cuda")
+        pi = np.array([N, A, k1 - k0, N, 1, 0, 0, 7, 0, 0], np.int32)
+        assert libraft.raft_fbp_device(0, _p(out), _p(x), _ptr(ang), _ptr(pf), _ptr(pi), 1, 1, None) == 0
+        return out
+
+    batch = run(0, n)
+    for k in (1, 2, 3):
+        assert torch.equal(run(0, k), batch[:k]), k
